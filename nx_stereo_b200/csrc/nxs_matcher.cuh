@@ -437,6 +437,23 @@ __device__ __forceinline__ uint32_t line_minimum(uint32_t v) {
     return v;
 }
 
+// The u16x2 minimum of a lane's words.
+template <int WORDS>
+__device__ __forceinline__ uint32_t words_minimum(const uint32_t (&w)[WORDS]) {
+    constexpr int PARTS = (WORDS + 2) / 3;
+    uint32_t part[PARTS];
+#pragma unroll
+    for (int k = 0; k < WORDS; k += 3)
+        part[k / 3] = k + 2 < WORDS ? __vimin3_u16x2(w[k], w[k + 1], w[k + 2])
+                                    : (k + 1 < WORDS ? vmin2(w[k], w[k + 1]) : w[k]);
+    uint32_t lowest = part[0];
+#pragma unroll
+    for (int k = 1; k < PARTS; k += 2)
+        lowest = k + 1 < PARTS ? __vimin3_u16x2(lowest, part[k], part[k + 1])
+                               : vmin2(lowest, part[k]);
+    return lowest;
+}
+
 // p + a * b bytes for a pointer p and 32-bit a, b, as one wide multiply-add.
 template <typename T>
 __device__ __forceinline__ T *advance(T *p, int a, unsigned b) {
@@ -445,22 +462,22 @@ __device__ __forceinline__ T *advance(T *p, int a, unsigned b) {
     return reinterpret_cast<T *>(d);
 }
 
-// The words of a permuted run (span_disparity) from its bytes, and back.
-__device__ __forceinline__ void unpack_run16(const uint4 c, uint32_t *w) {
-    w[0] = __byte_perm(c.x, 0, 0x4240);
-    w[1] = __byte_perm(c.x, 0, 0x4341);
-    w[2] = __byte_perm(c.y, 0, 0x4240);
-    w[3] = __byte_perm(c.y, 0, 0x4341);
-    w[4] = __byte_perm(c.z, 0, 0x4240);
-    w[5] = __byte_perm(c.z, 0, 0x4341);
-    w[6] = __byte_perm(c.w, 0, 0x4240);
-    w[7] = __byte_perm(c.w, 0, 0x4341);
+// The words of a permuted run (span_disparity) from its bytes, and back: the odd
+// word by a byte permute, the even one as c - 256 odd, a multiply-add by a run-time
+// -256 (FMA pipe), so half the unpacking leaves the integer pipe that bounds a step.
+__device__ __forceinline__ void unpack_pair(uint32_t c, uint32_t *w, uint32_t less_byte) {
+    w[1] = __byte_perm(c, 0, 0x4341);
+    w[0] = mad_lo(w[1], less_byte, c);
 }
-__device__ __forceinline__ void unpack_run8(const uint2 c, uint32_t *w) {
-    w[0] = __byte_perm(c.x, 0, 0x4240);
-    w[1] = __byte_perm(c.x, 0, 0x4341);
-    w[2] = __byte_perm(c.y, 0, 0x4240);
-    w[3] = __byte_perm(c.y, 0, 0x4341);
+__device__ __forceinline__ void unpack_run16(const uint4 c, uint32_t *w, uint32_t less_byte) {
+    unpack_pair(c.x, w, less_byte);
+    unpack_pair(c.y, w + 2, less_byte);
+    unpack_pair(c.z, w + 4, less_byte);
+    unpack_pair(c.w, w + 6, less_byte);
+}
+__device__ __forceinline__ void unpack_run8(const uint2 c, uint32_t *w, uint32_t less_byte) {
+    unpack_pair(c.x, w, less_byte);
+    unpack_pair(c.y, w + 2, less_byte);
 }
 // Halves below 256: w[2q] + 256 w[2q + 1] interleaves their bytes (a
 // multiply-add by a run-time 256, on the FMA pipe).
@@ -545,6 +562,22 @@ __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_gr
 template <int N>
 __device__ __forceinline__ void copy_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
+// Streaming stores under a predicate (evict first: the volumes do not fit the L2).
+__device__ __forceinline__ void store16_if(bool write, void *global, const uint4 v) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.u32 p, %0, 0;\n"
+        "@p st.global.cs.v4.u32 [%1], {%2, %3, %4, %5};\n}\n" ::"r"((unsigned)write),
+        "l"(global), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+        : "memory");
+}
+__device__ __forceinline__ void store8_if(bool write, void *global, const uint2 v) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.u32 p, %0, 0;\n@p st.global.cs.v2.u32 [%1], {%2, %3};\n}\n" ::
+            "r"((unsigned)write),
+        "l"(global), "r"(v.x), "r"(v.y)
+        : "memory");
 }
 
 // Adds four u16x2 words (eight u16 values below 1024) into 16 bytes of an
@@ -667,83 +700,56 @@ __host__ __device__ constexpr int sum_position(int disparities, int j) {
 // each stage completing on its own barrier of `bars` (LINES arrivals a
 // phase); the other blocks (each line's last ones) keep the per-lane copies,
 // their ring in the first stage's room once every tile has been read.
-template <int G, int WORDS, bool FULL, int THREADS, int SPAN = 0, bool SUMS = false,
-          bool TILES = false>
-__device__ __forceinline__ void follow_lines(const uint8_t *__restrict__ costs,
-                                             uint8_t *__restrict__ out, const PathSetup &s,
-                                             int p, int line, int member, void *ring_base,
-                                             const CostMaps *maps = nullptr,
-                                             uint8_t *tiles = nullptr, uint64_t *bars = nullptr) {
-    static_assert(WORDS == 4 || WORDS == 8 || WORDS == 16, "4, 8 or 16 words a lane");
-    static_assert(SPAN == 0 || (SPAN >= 8 && SPAN <= 2 * WORDS && (2 * WORDS) % SPAN == 0),
-                  "a lane holds whole permuted runs");
-    static_assert(!SUMS || WORDS == 8, "the aggregate layout has 16 disparities a lane");
-    static_assert(!TILES || (WORDS == 8 && SPAN == 16 && FULL), "tiles of 16 bytes a lane");
-    constexpr int BYTES = 2 * WORDS;             // a lane's disparities, one byte each
-    constexpr int PIECE = BYTES < 16 ? BYTES : 16;  // bytes of one async copy
-    constexpr int PIECES = BYTES / PIECE;
-    constexpr int RUN = SPAN / 2;                // words of a permuted run
-    constexpr int LINES = 32 / G;                // lines of a warp
+// The state of one scan line as a lane holds it, and its step.
+template <int G, int WORDS, bool FULL, int SPAN, bool SUMS>
+struct LineScan {
+    static constexpr int RUN = SPAN / 2;  // words of a permuted run
+    static constexpr int BYTES = 2 * WORDS;
+    static constexpr int PIECE = BYTES < 16 ? BYTES : 16;  // bytes of one copy or load
+    static constexpr int PIECES = BYTES / PIECE;
     using Piece = typename std::conditional<PIECE == 16, uint4, uint2>::type;
-    Piece *ring = static_cast<Piece *>(ring_base);
-    const int dy = s.dy[p], dx = s.dx[p];
-    const int W = s.width, H = s.height, D = s.disparities;
-    int y0 = 0, x0 = 0, length = 0;
-    if (line < s.lines[p]) length = line_start(line, dy, dx, W, H, &y0, &x0);
-    const bool active = FULL || member * BYTES < D;
-    const ptrdiff_t stride = ((ptrdiff_t)dy * W + dx) * D;  // |stride| <= 4097 x 256
-    const int stride32 = (int)stride;
-    const size_t at = ((size_t)y0 * W + x0) * D + member * BYTES;
-    const uint8_t *ahead = costs + at;
-    // SUMS: lane `member`'s words 0-3 at u16 (pixel * D + 8 * member), 4-7 D bytes on.
-    uint8_t *dst = SUMS ? out + 2 * (((size_t)y0 * W + x0) * D + 8 * member)
-                        : out + (size_t)p * s.volume + at;
-    const int steps = (int)__reduce_max_sync(kFullMask, (unsigned)length);
-    const int shortest = (int)__reduce_min_sync(kFullMask, (unsigned)length);
-    // Blocks all of whose steps every line of the warp has, with the copies they
-    // start (kPrefetch - 1 steps ahead), run without the checks: all blocks of the
-    // rows and columns but the last, most of each diagonal's.
-    auto unchecked_at = [&](int base) { return FULL && base + 2 * kPrefetch - 1 <= shortest; };
 
     uint32_t r[WORDS];
-#pragma unroll
-    for (int k = 0; k < WORDS; ++k) r[k] = active ? 0u : kInf2;
-    uint32_t m2 = 0, j2 = (uint32_t)s.p2 * 0x10001u;
-    const uint32_t p1x2 = (uint32_t)s.p1 * 0x10001u, p2x2 = (uint32_t)s.p2 * 0x10001u;
-    const uint32_t keep_left = member == 0 ? 0u : s.one, edge_left = member == 0 ? kInf2 : 0u;
-    const uint32_t keep_right = member == G - 1 ? 0u : s.one;
-    const uint32_t edge_right = member == G - 1 ? kInf2 : 0u;
-    const uint32_t byte = s.one << 8;  // 256, at run time (pack_run16)
+    uint32_t m2, j2;  // the line's lowest cost, and a jump from it, in both halves
+    uint32_t p1x2, p2x2, edge_left, edge_right, one, byte, less_byte;
+    int D;
 
-    auto fetch = [&](int slot, bool valid) {
+    __device__ __forceinline__ void begin(const PathSetup &s, int member, bool active) {
+        // Lanes past the line's disparities stay far above every cost by their own
+        // penalties.
+#pragma unroll
+        for (int k = 0; k < WORDS; ++k) r[k] = active ? 0u : kInf2;
+        p1x2 = active ? (uint32_t)s.p1 * 0x10001u : kInf2;
+        p2x2 = active ? (uint32_t)s.p2 * 0x10001u : kFar2;
+        m2 = 0;
+        j2 = p2x2;
+        one = s.one;
+        byte = s.one << 8;  // 256, at run time (pack_run16)
+        less_byte = 0u - byte;
+        edge_left = member == 0 ? kInf2 : 0u;
+        edge_right = member == G - 1 ? kInf2 : 0u;
+        D = s.disparities;
+    }
+
+    __device__ __forceinline__ void unpack(const Piece *from, int stride, uint32_t (&cost)[WORDS]) const {
 #pragma unroll
         for (int c = 0; c < PIECES; ++c) {
-            Piece *to = ring + (slot * PIECES + c) * THREADS;
-            const uint8_t *from = valid ? ahead + PIECE * c : costs;
-            if (PIECE == 16) copy16_async(to, from, valid);
-            else copy8_async(to, from, valid);
+            if constexpr (PIECE == 16) {
+                if constexpr (SPAN != 0) unpack_run16(from[c * stride], cost + 8 * c, less_byte);
+                else unpack16(from[c * stride], cost + 8 * c);
+            } else {
+                if constexpr (SPAN != 0) unpack_run8(from[c * stride], cost + 4 * c, less_byte);
+                else unpack8(from[c * stride], cost + 4 * c);
+            }
         }
-        copy_commit();
-        ahead = advance(ahead, stride32, s.one);
-    };
-    // The ring's first kPrefetch - 1 slots take steps base .. base + kPrefetch - 2.
-    auto prime = [&](int base) {
-        ahead = costs + at + (ptrdiff_t)base * stride;
-#pragma unroll
-        for (int i = 0; i < kPrefetch - 1; ++i) fetch(i, active && base + i < length);
-    };
-    if (!(TILES && unchecked_at(0))) prime(0);
+    }
 
-    // One step from this step's costs: the recurrence on every word, the
-    // store (or reduction) of the path costs where `store`, the line's minimum.
-    auto advance_step = [&](const uint32_t(&cost)[WORDS], bool store) {
-        // The line's first and last lanes see +inf past the ends: x keep + edge
-        // as multiply-adds (keep 0 and edge kInf2 there, 1 and 0 elsewhere).
-        const uint32_t from_left =
-            mad_lo(__shfl_up_sync(kFullMask, r[WORDS - 1], 1), keep_left, edge_left);
-        const uint32_t from_right =
-            mad_lo(__shfl_down_sync(kFullMask, r[0], 1), keep_right, edge_right);
-        const uint32_t negm2 = 0u - m2;
+    // One step from this step's costs: the recurrence on every word, the store (or
+    // reduction) of the path costs where `store`, the line's minimum.
+    __device__ __forceinline__ void step(const uint32_t (&cost)[WORDS], uint8_t *dst, bool store) {
+        // The line's first and last lanes see +inf past the ends (add2 with kInf2).
+        const uint32_t from_left = add2(__shfl_up_sync(kFullMask, r[WORDS - 1], 1), edge_left);
+        const uint32_t from_right = add2(__shfl_down_sync(kFullMask, r[0], 1), edge_right);
         uint32_t below[WORDS], above[WORDS];  // word k's values at d - 1 and at d + 1
         if constexpr (SPAN != 0) {
 #pragma unroll
@@ -771,87 +777,119 @@ __device__ __forceinline__ void follow_lines(const uint8_t *__restrict__ costs,
                 above[k] = shifted[k + 1];
             }
         }
+        const uint32_t negm2 = 0u - m2;
 #pragma unroll
         for (int k = 0; k < WORDS; ++k) {
-            // min(prev, neighbours + p1, m + p2) - m + cost: neighbours + p1
-            // (a multiply-add by a run-time 1, on the FMA pipe beside the
-            // integer pipe's min and permute work) <= 0x7FFF + 79 stays in its
-            // half; t + cost + (-m) is one three-input add taken mod 2^32,
-            // which equals t - m + cost, whose halves neither borrow nor carry
-            // (t >= m in both). It measured 3% faster than two multiply-adds.
+            // min(prev, neighbours + p1, m + p2) - m + cost: the sum is one three-input
+            // add taken mod 2^32, whose halves neither borrow nor carry (t >= m in both).
             const uint32_t neighbour = vmin2(below[k], above[k]);
-            const uint32_t raised = mad_lo(neighbour, s.one, p1x2);
-            const uint32_t t = __vimin3_u16x2(r[k], j2, raised);
-            const uint32_t value = t + cost[k] + negm2;
-            r[k] = (FULL || active) ? value : kInf2;
+            const uint32_t raised = add2(neighbour, p1x2);
+            const uint32_t t = __vimin3_u16x2(r[k], raised, j2);
+            r[k] = t + cost[k] + negm2;
         }
-        if (store) {
-            if constexpr (SUMS) {
+        const uint32_t lowest = words_minimum<WORDS>(r);
+        m2 = line_minimum<G>(vmin2(lowest, __byte_perm(lowest, 0, 0x1032)));
+        j2 = add2(m2, p2x2);
+        if constexpr (SUMS) {
+            if (store) {
                 add_sums16(dst, r[0], r[1], r[2], r[3]);
                 add_sums16(dst + D, r[4], r[5], r[6], r[7]);
-            } else {
+            }
+        } else {
+            // The bytes first, then a predicated store: a branch around the packing too
+            // costs every step its resolution.
 #pragma unroll
-                for (int c = 0; c < PIECES; ++c) {
-                    if constexpr (PIECE == 16)
-                        __stcs(reinterpret_cast<uint4 *>(dst + 16 * c),
+            for (int c = 0; c < PIECES; ++c) {
+                if constexpr (PIECE == 16)
+                    store16_if(store, dst + 16 * c,
                                SPAN ? pack_run16(r + 8 * c, byte) : pack16(r + 8 * c));
-                    else
-                        __stcs(reinterpret_cast<uint2 *>(dst + 8 * c),
-                               SPAN ? pack_run8(r + 4 * c, byte) : pack8(r + 4 * c));
-                }
+                else
+                    store8_if(store, dst + 8 * c,
+                              SPAN ? pack_run8(r + 4 * c, byte) : pack8(r + 4 * c));
             }
         }
-        dst = advance(dst, SUMS ? 2 * stride32 : stride32, s.one);
-        // The lowest path cost over the line's disparities: a shallow tree
-        // over the lane's words, both halves folded into each half, then
-        // over the line's G lanes a shuffle tree (one warp-wide reduction
-        // when the line has the whole warp; a reduction under each group's
-        // own mask measured slower than the shuffles).
-        constexpr int PARTS = (WORDS + 2) / 3;
-        uint32_t part[PARTS];
+    }
+};
+
+template <int G, int WORDS, bool FULL, int THREADS, int SPAN = 0, bool SUMS = false,
+          bool TILES = false, int RING = kPrefetch>
+__device__ __forceinline__ void follow_lines(const uint8_t *__restrict__ costs,
+                                             uint8_t *__restrict__ out, const PathSetup &s,
+                                             int p, int line, bool own, int member,
+                                             void *ring_base,
+                                             const CostMaps *maps = nullptr,
+                                             uint8_t *tiles = nullptr, uint64_t *bars = nullptr) {
+    static_assert(WORDS == 4 || WORDS == 8 || WORDS == 16, "4, 8 or 16 words a lane");
+    static_assert(SPAN == 0 || (SPAN >= 8 && SPAN <= 2 * WORDS && (2 * WORDS) % SPAN == 0),
+                  "a lane holds whole permuted runs");
+    static_assert(!SUMS || WORDS == 8, "the aggregate layout has 16 disparities a lane");
+    static_assert(!TILES || RING == kPrefetch, "a block of steps is a tile");
+    static_assert(!TILES || (WORDS == 8 && SPAN == 16 && FULL), "tiles of 16 bytes a lane");
+    using Scan = LineScan<G, WORDS, FULL, SPAN, SUMS>;
+    using Piece = typename Scan::Piece;
+    constexpr int BYTES = Scan::BYTES, PIECE = Scan::PIECE, PIECES = Scan::PIECES;
+    constexpr int LINES = 32 / G;                // lines of a warp
+    Piece *ring = static_cast<Piece *>(ring_base);
+    const int dy = s.dy[p], dx = s.dx[p];
+    const int W = s.width, H = s.height, D = s.disparities;
+    int y0 = 0, x0 = 0;
+    const int length = line_start(line, dy, dx, W, H, &y0, &x0);
+    const bool active = FULL || member * BYTES < D, writes = own && active;
+    const ptrdiff_t stride = ((ptrdiff_t)dy * W + dx) * D;  // |stride| <= 4097 x 256
+    const int stride32 = (int)stride, dst_stride = SUMS ? 2 * stride32 : stride32;
+    // Lanes past the disparities read the line's first ones, and write nothing.
+    const size_t at = ((size_t)y0 * W + x0) * D + (active ? member * BYTES : 0);
+    const uint8_t *ahead = costs + at;
+    // SUMS: lane `member`'s words 0-3 at u16 (pixel * D + 8 * member), 4-7 D bytes on.
+    uint8_t *dst = SUMS ? out + 2 * (((size_t)y0 * W + x0) * D + 8 * member)
+                        : out + (size_t)p * s.volume + at;
+    const int steps = (int)__reduce_max_sync(kFullMask, (unsigned)length);
+    const int shortest = (int)__reduce_min_sync(kFullMask, (unsigned)length);
+    // Blocks all of whose steps every line of the warp has, with the copies they
+    // start (RING - 1 steps ahead), run without the checks: all blocks of the
+    // rows and columns but the last, most of each diagonal's.
+    auto unchecked_at = [&](int base) { return base + 2 * RING - 1 <= shortest; };
+
+    Scan scan;
+    scan.begin(s, member, active);
+
+    auto fetch = [&](int slot, bool valid) {
 #pragma unroll
-        for (int k = 0; k < WORDS; k += 3)
-            part[k / 3] = k + 2 < WORDS ? __vimin3_u16x2(r[k], r[k + 1], r[k + 2])
-                                        : (k + 1 < WORDS ? vmin2(r[k], r[k + 1]) : r[k]);
-        uint32_t lowest = part[0];
-#pragma unroll
-        for (int k = 1; k < PARTS; k += 2)
-            lowest = k + 1 < PARTS ? __vimin3_u16x2(lowest, part[k], part[k + 1])
-                                   : vmin2(lowest, part[k]);
-        lowest = vmin2(lowest, __byte_perm(lowest, 0, 0x1032));
-        if constexpr (G == 32) {
-            m2 = __reduce_min_sync(kFullMask, lowest);
-        } else {
-            lowest = line_minimum<G>(lowest);
-            m2 = lowest;
+        for (int c = 0; c < PIECES; ++c) {
+            Piece *to = ring + (slot * PIECES + c) * THREADS;
+            const uint8_t *from = valid ? ahead + PIECE * c : costs;
+            if (PIECE == 16) copy16_async(to, from, valid);
+            else copy8_async(to, from, valid);
         }
-        j2 = m2 + p2x2;
+        copy_commit();
+        ahead = advance(ahead, stride32, s.one);
     };
-    // One block of kPrefetch steps from `base` from the ring. CHECKED: the steps
+    // The ring's first RING - 1 slots take steps base .. base + RING - 2.
+    auto prime = [&](int base) {
+        ahead = costs + at + (ptrdiff_t)base * stride;
+#pragma unroll
+        for (int i = 0; i < RING - 1; ++i) fetch(i, base + i < length);
+    };
+    if (!(TILES && unchecked_at(0))) prime(0);
+
+    // One block of RING steps from `base` from the ring. CHECKED: the steps
     // test the warp's last step and each line's end; without, every line of the
     // warp covers the block and the copies it starts (FULL: every lane active).
     auto block = [&](const int base, auto checked) {
         constexpr bool CHECKED = decltype(checked)::value;
 #pragma unroll
-        for (int i = 0; i < kPrefetch; ++i) {
+        for (int i = 0; i < RING; ++i) {
             const int step = base + i;
             if (CHECKED && step >= steps) break;  // uniform across the warp
-            // the copy of step + kPrefetch - 1 goes to the slot read last step
-            fetch((i + kPrefetch - 1) % kPrefetch,
-                  !CHECKED || (active && step + kPrefetch - 1 < length));
-            copy_wait<kPrefetch - 1>();
+            // the copy of step + RING - 1 goes to the slot read last step
+            fetch((i + RING - 1) % RING,
+                  !CHECKED || step + RING - 1 < length);
+            copy_wait<RING - 1>();
             uint32_t cost[WORDS];
-#pragma unroll
-            for (int c = 0; c < PIECES; ++c) {
-                if constexpr (PIECE == 16) {
-                    if constexpr (SPAN != 0) unpack_run16(ring[(i * PIECES + c) * THREADS], cost + 8 * c);
-                    else unpack16(ring[(i * PIECES + c) * THREADS], cost + 8 * c);
-                } else {
-                    if constexpr (SPAN != 0) unpack_run8(ring[(i * PIECES + c) * THREADS], cost + 4 * c);
-                    else unpack8(ring[(i * PIECES + c) * THREADS], cost + 4 * c);
-                }
-            }
-            advance_step(cost, !CHECKED || (active && step < length));
+            scan.unpack(ring + i * PIECES * THREADS, THREADS, cost);
+            const bool store = writes && (!CHECKED || step < length);
+            scan.step(cost, dst, store);
+            dst = advance(dst, dst_stride, s.one);
         }
     };
 
@@ -895,15 +933,17 @@ __device__ __forceinline__ void follow_lines(const uint8_t *__restrict__ costs,
 #pragma unroll
                 for (int i = 0; i < kPrefetch; ++i) {
                     uint32_t cost[WORDS];
-                    unpack_run16(tile[i * G], cost);
-                    advance_step(cost, true);
+                    scan.unpack(tile + i * G, 1, cost);
+                    scan.step(cost, dst, writes);
+                    dst = advance(dst, dst_stride, s.one);
                 }
             } else {
 #pragma unroll
                 for (int i = 0; i < kPrefetch; ++i) {
                     uint32_t cost[WORDS];
-                    unpack_run16(tile[(kPrefetch - 1 - i) * G], cost);
-                    advance_step(cost, true);
+                    scan.unpack(tile + (kPrefetch - 1 - i) * G, 1, cost);
+                    scan.step(cost, dst, writes);
+                    dst = advance(dst, dst_stride, s.one);
                 }
             }
         }
@@ -915,7 +955,7 @@ __device__ __forceinline__ void follow_lines(const uint8_t *__restrict__ costs,
             block(base, std::true_type());
         }
     } else {
-        for (int base = 0; base < steps; base += kPrefetch) {
+        for (int base = 0; base < steps; base += RING) {
             if (unchecked_at(base)) block(base, std::false_type());
             else block(base, std::true_type());
         }
@@ -952,7 +992,8 @@ __host__ __device__ __forceinline__ int ranked_line(int rank, int dy, int dx, in
 // Rows, then columns, then the diagonals of all four directions by rank.
 // `ring`: this lane's first slot of the warp's kPrefetch x 32 slots of
 // 2 x WORDS bytes (in pieces of at most 16 bytes, strided by 32 lanes).
-template <int G, int WORDS, bool FULL, int SPAN = 0, bool SUMS = false, bool TILES = false>
+template <int G, int WORDS, bool FULL, int SPAN = 0, bool SUMS = false, bool TILES = false,
+          int RING = kPrefetch>
 __device__ __forceinline__ void path_warp(const uint8_t *__restrict__ costs,
                                           uint8_t *__restrict__ paths_out, const PathSetup &s,
                                           int warp, int lane, void *ring,
@@ -970,11 +1011,15 @@ __device__ __forceinline__ void path_warp(const uint8_t *__restrict__ costs,
         p = s.order[s.straight + w % diagonals];
         group = w / diagonals;
     }
-    const int rank = group * (32 / G) + lane / G;
-    const int line =
-        rank < s.lines[p] ? ranked_line(rank, s.dy[p], s.dx[p], s.width, s.height) : rank;
-    follow_lines<G, WORDS, FULL, 32, SPAN, SUMS, TILES>(costs, paths_out, s, p, line, lane % G,
-                                                        ring, maps, tiles, bars);
+    // The last warp of a direction follows its last line again, without writing, in the
+    // groups that have none of their own: a group without a line would take the whole
+    // warp through the steps' checks (480x270x64, 3 paths: 270 rows are 33.75 warps, and
+    // the ragged one alone set the kernel's time).
+    const int own = group * (32 / G) + lane / G;
+    const int rank = min(own, s.lines[p] - 1);
+    const int line = ranked_line(rank, s.dy[p], s.dx[p], s.width, s.height);
+    follow_lines<G, WORDS, FULL, 32, SPAN, SUMS, TILES, RING>(
+        costs, paths_out, s, p, line, own < s.lines[p], lane % G, ring, maps, tiles, bars);
 }
 
 // Lanes per pixel (selection) or per line (paths with 16 disparities a lane),
