@@ -109,13 +109,19 @@ cudaError_t launch_census_costs(const uint8_t *left, const uint8_t *right, int w
 // TILES: the blocks of steps every line of a warp covers take their costs by
 // bulk tensor copies of `maps` into kTileStages stages of 8 steps x 32 lanes
 // x 16 bytes; the per-lane ring of the other steps shares the first stage.
+// kPathRing: steps of costs a lane keeps in flight by its own copies. 12 cover the L2's
+// latency under the streaming stores (1277x713x192 with 3 paths 485 us a pair, 499 with 8;
+// 16 gave no more), at 6 KB of shared memory a block.
+constexpr int kPathRing = 12;
+
 template <int G, int WORDS, bool FULL, int SPAN, bool SUMS = false, bool TILES = false>
 __global__ void __launch_bounds__(32)
     paths_kernel(const uint8_t *__restrict__ costs, uint8_t *__restrict__ paths_out,
                  const PathSetup s, const __grid_constant__ CostMaps maps) {
     using Piece = typename std::conditional<WORDS == 4, uint2, uint4>::type;
     constexpr int PIECES = WORDS == 16 ? 2 : 1;
-    constexpr int RING_BYTES = kPrefetch * PIECES * 32 * (int)sizeof(Piece);
+    constexpr int RING = TILES ? kPrefetch : kPathRing;
+    constexpr int RING_BYTES = RING * PIECES * 32 * (int)sizeof(Piece);
     constexpr int TILE_BYTES = kTileStages * kPrefetch * 32 * 16;
     static_assert(!TILES || RING_BYTES <= TILE_BYTES / kTileStages, "the ring fits one stage");
     __shared__ __align__(128) uint8_t room[TILES ? TILE_BYTES : RING_BYTES];
@@ -128,9 +134,9 @@ __global__ void __launch_bounds__(32)
         __syncwarp();
     }
     follow_previous_grid();
-    path_warp<G, WORDS, FULL, SPAN, SUMS, TILES>(costs, paths_out, s, blockIdx.x, threadIdx.x,
-                                                 reinterpret_cast<Piece *>(room) + threadIdx.x,
-                                                 &maps, room, bars);
+    path_warp<G, WORDS, FULL, SPAN, SUMS, TILES, RING>(
+        costs, paths_out, s, blockIdx.x, threadIdx.x,
+        reinterpret_cast<Piece *>(room) + threadIdx.x, &maps, room, bars);
 }
 
 // ---- the cost volume's tensor maps (cuTensorMapEncodeTiled, from the driver) ----
@@ -268,7 +274,7 @@ static void launch_paths_in(const uint8_t *costs, uint8_t *paths_out, const Path
         if (full && tiles_wanted(s.width, s.height, s.disparities) &&
             encode_cost_maps(costs, s.width, s.height, s.disparities, &maps)) {
 #define NXS_TILED(G)                                                                           \
-    launch_after(paths_kernel<G, 8, true, 16, false, true>, dim3(total), dim3(32), 0, stream,  \
+    launch_carved<-1>(paths_kernel<G, 8, true, 16, false, true>, dim3(total), dim3(32), 0, stream, \
                  costs, paths_out, s, maps)
             if (g == 4) NXS_TILED(4);
             else if (g == 8) NXS_TILED(8);
@@ -450,7 +456,7 @@ static cudaError_t launch_select(const void *source, int width, int height, int 
         return cudaGetLastError();
     }
 #define NXS_SELECT(G)                                                                         \
-    launch_after(select_kernel<G, PATHS, SPAN>, dim3(blocks), dim3(128), 0, stream, source,   \
+    launch_carved<-1>(select_kernel<G, PATHS, SPAN>, dim3(blocks), dim3(128), 0, stream, source, \
                  width, height, disparities, volume, uniqueness, disparity, keys, 1u)
     if (g == 4) NXS_SELECT(4);
     else if (g == 8) NXS_SELECT(8);

@@ -61,20 +61,39 @@ __device__ __forceinline__ void follow_previous_grid() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-template <typename... Params, typename... Args>
-inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared,
-                                cudaStream_t stream, Args &&...args) {
+// CARVEOUT: the percentage of an SM's L1 memory a kernel asks for as shared memory (-1: the
+// driver's choice, by that kernel alone).
+template <int CARVEOUT, typename... Params, typename... Args>
+inline cudaError_t launch_carved(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared,
+                                 cudaStream_t stream, Args &&...args) {
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
     config.blockDim = block;
     config.dynamicSmemBytes = shared;
     config.stream = stream;
-    cudaLaunchAttribute attribute[1];
+    cudaLaunchAttribute attribute[2];
     attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attribute[0].val.programmaticStreamSerializationAllowed = 1;
+    attribute[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attribute[1].val.sharedMemCarveout = (unsigned)CARVEOUT;
     config.attrs = attribute;
-    config.numAttrs = 1;
+    config.numAttrs = CARVEOUT < 0 ? 1 : 2;
     return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
+}
+
+// The kernels that run beside one another (a segment's two lanes, a batch's streams) ask
+// for the same split of the L1: an SM that holds blocks of one split takes none of another,
+// so with the driver's choice for each kernel a path scan and a selection shut each other
+// out (four 1280x720x128 stream pairs 3,190 us, 2,951 with one split; 16 mixed pairs in a
+// batch 2,258 and 2,124). 60% (137 KB shared) holds 22 blocks of the path scan; the rest is
+// the room in which the selection's loads land: 40% and 100% measured 581 and 553 us for a
+// 1280x720x128 pair against 508.
+constexpr int kCarveout = 60;
+template <typename... Params, typename... Args>
+inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared,
+                                cudaStream_t stream, Args &&...args) {
+    return launch_carved<kCarveout>(kernel, grid, block, shared, stream,
+                                    std::forward<Args>(args)...);
 }
 
 }  // namespace nxs
