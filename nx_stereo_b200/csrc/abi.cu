@@ -1027,6 +1027,31 @@ extern "C" nxs_status nxs_despeckle_depth_cloud_device(
                : NXS_OK;
 }
 
+// The library's own stream-ordered pool on the current device, made on first use. It keeps
+// up to 32 MiB (the step a pool grows by) between calls: the device's default pool gives
+// everything back at each synchronisation, so that a call after one maps memory anew (a lone
+// pass of the stages at 1280x720 took 690 us, 500 of them that).
+static cudaMemPool_t small_pool() {
+    constexpr int kDevices = 64;
+    static std::mutex lock;
+    static cudaMemPool_t pools[kDevices] = {};
+    int device = 0;
+    if (cudaGetDevice(&device) || device < 0 || device >= kDevices) return nullptr;
+    std::lock_guard<std::mutex> guard(lock);
+    if (!pools[device]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props)) return nullptr;
+        uint64_t keep = 32u << 20;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        pools[device] = pool;
+    }
+    return pools[device];
+}
+
 extern "C" nxs_status nxs_quality_device(const float *d_disparity, float *d_previous,
                                          uint32_t width, uint32_t height, float *d_sums,
                                          void *stream) {
@@ -1034,7 +1059,9 @@ extern "C" nxs_status nxs_quality_device(const float *d_disparity, float *d_prev
     // The per-column sums live in a small stream-ordered allocation.
     float *columns = nullptr;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (cudaMallocAsync(reinterpret_cast<void **>(&columns), sizeof(float) * 5 * width, s))
+    const cudaMemPool_t pool = small_pool();
+    if (!pool || cudaMallocFromPoolAsync(reinterpret_cast<void **>(&columns),
+                                         sizeof(float) * 5 * width, pool, s))
         return NXS_CUDA_ERROR;
     cudaError_t e = launch_quality(d_disparity, d_previous, width, height, columns, d_sums, s);
     cudaFreeAsync(columns, s);

@@ -499,53 +499,83 @@ cudaError_t launch_despeckle_depth_cloud(const float *disparity, int width, int 
 }
 
 // ---------------------------------------------------------------- quality
-// lib/nx_stereo/diagnostics.ex:264-271 with the native reduction order
+// lib/nx_stereo/diagnostics.ex:264-271 with the native reduction's precision
 // (native/stereo_match/src/measures.rs:278-309): per column, the five planes
-// [matched, value, value^2, both, |change| * both] summed down the rows in
-// f64 and rounded to f32; then the columns summed in order in f64 and
-// rounded. One thread per column, then one per plane.
-__global__ void quality_columns_kernel(const float *__restrict__ disparity,
-                                       const float *__restrict__ previous, int width, int height,
-                                       float *__restrict__ column_sums) {
+// [matched, value, value^2, both, |change| * both] summed over the rows in
+// f64 and rounded to f32; then the columns' sums summed in f64 and rounded.
+//
+// A block takes kQualityX columns (a 32-byte sector of a row) with kQualityRows threads down
+// each: every thread sums every kQualityRows-th row of its column, so a column is 64 short
+// chains instead of one of H dependent steps, and 1280 columns are 160 blocks of 512 instead
+// of 10 of 128. The f64 partial sums are then added in a fixed order. The kernel also moves
+// the disparity into `previous`, both being in hand, which was a copy of its own.
+constexpr int kQualityX = 8, kQualityRows = 64, kQualityWarps = kQualityX * kQualityRows / 32;
+
+__global__ void __launch_bounds__(kQualityX *kQualityRows)
+    quality_columns_kernel(const float *__restrict__ disparity, float *__restrict__ previous,
+                           int width, int height, float *__restrict__ column_sums) {
     follow_previous_grid();
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= width) return;
+    __shared__ double partial[kQualityWarps][5][kQualityX];
+    const int column = threadIdx.x % kQualityX, x = blockIdx.x * kQualityX + column;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     double acc[5] = {0, 0, 0, 0, 0};
-    for (int y = 0; y < height; ++y) {
-        const float current = disparity[(size_t)y * width + x];
-        const float before = previous[(size_t)y * width + x];
-        const float matched = current > 0.0f ? 1.0f : 0.0f;
-        const float both = fmul(before > 0.0f ? 1.0f : 0.0f, matched);
-        const float value = fmul(current, matched);
-        acc[0] += (double)matched;
-        acc[1] += (double)value;
-        acc[2] += (double)fmul(value, value);
-        acc[3] += (double)both;
-        acc[4] += (double)fmul(fabsf(fsub(current, before)), both);
+    if (x < width) {
+#pragma unroll 4
+        for (int y = threadIdx.x / kQualityX; y < height; y += kQualityRows) {
+            const size_t i = (size_t)y * width + x;
+            const float current = disparity[i], before = previous[i];
+            const float matched = current > 0.0f ? 1.0f : 0.0f;
+            const float both = fmul(before > 0.0f ? 1.0f : 0.0f, matched);
+            const float value = fmul(current, matched);
+            acc[0] += (double)matched;
+            acc[1] += (double)value;
+            acc[2] += (double)fmul(value, value);
+            acc[3] += (double)both;
+            acc[4] += (double)fmul(fabsf(fsub(current, before)), both);
+            previous[i] = current;
+        }
     }
+    // A warp's four rows of the columns, then the warps'.
 #pragma unroll
-    for (int p = 0; p < 5; ++p) column_sums[(size_t)p * width + x] = (float)acc[p];
+    for (int p = 0; p < 5; ++p) {
+#pragma unroll
+        for (int offset = 16; offset >= kQualityX; offset /= 2)
+            acc[p] += __shfl_down_sync(kFullMask, acc[p], offset);
+        if (lane < kQualityX) partial[warp][p][lane] = acc[p];
+    }
+    __syncthreads();
+    const int p = threadIdx.x / kQualityX;  // the plane this thread adds up for its column
+    if (p >= 5 || x >= width) return;
+    double total = 0.0;
+#pragma unroll
+    for (int w = 0; w < kQualityWarps; ++w) total += partial[w][p][column];
+    column_sums[(size_t)p * width + x] = (float)total;
 }
 
-__global__ void quality_total_kernel(const float *__restrict__ column_sums, int width,
-                                     float *__restrict__ sums) {
+// One warp a plane: every lane sums every 32nd column, then the lanes' sums are added by
+// halves (one thread a plane, W dependent steps, took 26 us at 1280 columns).
+__global__ void __launch_bounds__(5 * 32)
+    quality_total_kernel(const float *__restrict__ column_sums, int width,
+                         float *__restrict__ sums) {
     follow_previous_grid();
-    const int p = threadIdx.x;
-    if (p >= 5) return;
+    const int p = threadIdx.x / 32, lane = threadIdx.x % 32;
     double total = 0.0;
-    for (int x = 0; x < width; ++x) total += (double)column_sums[(size_t)p * width + x];
-    sums[p] = (float)total;
+#pragma unroll 8
+    for (int x = lane; x < width; x += 32) total += (double)column_sums[(size_t)p * width + x];
+#pragma unroll
+    for (int offset = 16; offset >= 1; offset /= 2)
+        total += __shfl_down_sync(kFullMask, total, offset);
+    if (lane == 0) sums[p] = (float)total;
 }
 
 cudaError_t launch_quality(const float *disparity, float *previous, int width, int height,
                            float *column_sums, float *sums, cudaStream_t stream) {
-    cudaError_t e = launch_after(quality_columns_kernel, dim3((width + 127) / 128), dim3(128), 0,
-                                 stream, disparity, previous, width, height, column_sums);
-    if (!e) e = launch_after(quality_total_kernel, dim3(1), dim3(32), 0, stream, column_sums,
-                             width, sums);
+    const cudaError_t e = launch_after(
+        quality_columns_kernel, dim3((width + kQualityX - 1) / kQualityX),
+        dim3(kQualityX * kQualityRows), 0, stream, disparity, previous, width, height, column_sums);
     if (e) return e;
-    return cudaMemcpyAsync(previous, disparity, sizeof(float) * (size_t)width * height,
-                           cudaMemcpyDeviceToDevice, stream);
+    return launch_after(quality_total_kernel, dim3(1), dim3(5 * 32), 0, stream, column_sums,
+                        width, sums);
 }
 
 }  // namespace nxs
