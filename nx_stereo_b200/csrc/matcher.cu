@@ -396,30 +396,30 @@ cudaError_t launch_sum_paths(const uint8_t *paths_in, int width, int height, int
 
 // ---------------------------------------------------------------- select
 // `one` is 1, given at run time (select_pixels adds by multiply-adds).
-template <int G, int PATHS, int SPAN>
+template <int G, int PATHS, int SPAN, int RUNS>
 __global__ void __launch_bounds__(128)
     select_kernel(const void *__restrict__ source, int width, int height, int disparities,
                   size_t volume, float uniqueness, float *__restrict__ disparity,
                   uint32_t *__restrict__ keys, uint32_t one) {
     follow_previous_grid();
-    __shared__ __align__(16) uint16_t values_of[128 / G][256];
-    select_pixels<G, PATHS, SPAN>(source, width, height, disparities, volume, uniqueness,
+    __shared__ __align__(16) uint16_t values_of[128 / G][RUNS == 1 ? 256 : 16 * G * RUNS];
+    select_pixels<G, PATHS, SPAN, RUNS>(source, width, height, disparities, volume, uniqueness,
                                   disparity, keys, nullptr, blockIdx.x, values_of, one);
 }
 
 // select_kernel with a grid of `resident` blocks that step through the
 // pixel blocks: a selection run beside another stream's path scan holds
 // fewer warps a SM while it streams the path volumes.
-template <int G, int PATHS, int SPAN>
+template <int G, int PATHS, int SPAN, int RUNS>
 __global__ void __launch_bounds__(128)
     select_lean_kernel(const void *__restrict__ source, int width, int height, int disparities,
                        size_t volume, float uniqueness, float *__restrict__ disparity,
                        uint32_t *__restrict__ keys, uint32_t one, size_t blocks) {
     follow_previous_grid();
-    __shared__ __align__(16) uint16_t values_of[128 / G][256];
+    __shared__ __align__(16) uint16_t values_of[128 / G][RUNS == 1 ? 256 : 16 * G * RUNS];
     for (size_t block = blockIdx.x; block < blocks; block += gridDim.x) {
         __syncwarp();  // the group's row of values_of is read before it is rewritten
-        select_pixels<G, PATHS, SPAN>(source, width, height, disparities, volume, uniqueness,
+        select_pixels<G, PATHS, SPAN, RUNS>(source, width, height, disparities, volume, uniqueness,
                                       disparity, keys, nullptr, block, values_of, one);
     }
 }
@@ -432,35 +432,71 @@ static std::atomic<int> g_lean_select{8};
 void set_lean_select(int blocks_per_sm) { g_lean_select = blocks_per_sm < 0 ? 0 : blocks_per_sm; }
 int lean_select() { return g_lean_select.load(); }
 
+// Runs of 16 disparities a selection lane takes. One run a lane spends two rounds of
+// log2(D / 16) shuffles and the winner's f32 steps on few volumes' bytes: three volumes are
+// too few to hide that, and with 96 or 192 disparities a quarter of the lanes idle. More
+// runs a lane measured (us, one run -> this table): 3 paths 1280x720x64 52.9 -> 39.4, x128
+// 87.3 -> 72.0, x256 174.8 -> 134.5 (two runs 146.1), 641x479x96 30.1 -> 18.0, 1277x713x192
+// 171.0 -> 104.2; 8 paths 1280x720x64 92.8 -> 79.7. With 8 paths that is so only at 64
+// disparities and above half a million pixels: the smaller frames stay in L2 and want the
+// warps (364x272x64 within a coarse-to-fine pair 176.5 us, 178.4 with two runs; a lean grid
+// in a batch 2,119 and 2,150), and with more disparities the volumes' bytes bound it, which
+// fewer lanes a pixel read in smaller pieces (728x544x128 61.7, 69.3 with two runs;
+// 641x479x96 44.8, 77.4 with three).
+static int select_runs(int disparities, int paths, size_t pixels, bool lean) {
+    if (paths == 8) return disparities == 64 && !lean && pixels >= ((size_t)1 << 19) ? 2 : 1;
+    if (paths != 3) return 1;
+    switch (disparities) {
+    case 64: case 128: return 2;
+    case 96: case 192: return 3;
+    case 256: return 4;
+    default: return 1;
+    }
+}
+
 template <int PATHS, int SPAN = 0>
 static cudaError_t launch_select(const void *source, int width, int height, int disparities,
                                  float uniqueness, float *disparity, uint32_t *keys,
                                  cudaStream_t stream, int lean = 0) {
     const size_t pixels = (size_t)width * height;
     const size_t volume = pixels * disparities;
-    const int g = group_lanes(disparities);
+    const int runs = select_runs(disparities, PATHS, pixels, lean > 0);
+    const int g = runs == 1 ? group_lanes(disparities) : disparities / (16 * runs);
     const unsigned blocks = (unsigned)((pixels + 128 / g - 1) / (128 / g));
     if (lean > 0) {
         int device = 0, sms = 148;
         cudaGetDevice(&device);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         const unsigned grid = std::min<unsigned>(blocks, (unsigned)(lean * sms));
-#define NXS_LEAN(G)                                                                            \
-    launch_after(select_lean_kernel<G, PATHS, SPAN>, dim3(grid), dim3(128), 0, stream, source,  \
+#define NXS_LEAN(G, R)                                                                         \
+    launch_after(select_lean_kernel<G, PATHS, SPAN, R>, dim3(grid), dim3(128), 0, stream, source,  \
                  width, height, disparities, volume, uniqueness, disparity, keys, 1u,           \
                  (size_t)blocks)
-        if (g == 4) NXS_LEAN(4);
-        else if (g == 8) NXS_LEAN(8);
-        else NXS_LEAN(16);
+        if constexpr (PATHS == 3) {
+            if (runs == 2) return g == 2 ? NXS_LEAN(2, 2) : NXS_LEAN(4, 2);
+            if (runs == 3) return g == 2 ? NXS_LEAN(2, 3) : NXS_LEAN(4, 3);
+            if (runs == 4) return NXS_LEAN(4, 4);
+        }
+        if (g == 4) NXS_LEAN(4, 1);
+        else if (g == 8) NXS_LEAN(8, 1);
+        else NXS_LEAN(16, 1);
 #undef NXS_LEAN
         return cudaGetLastError();
     }
-#define NXS_SELECT(G)                                                                         \
-    launch_carved<-1>(select_kernel<G, PATHS, SPAN>, dim3(blocks), dim3(128), 0, stream, source, \
+#define NXS_SELECT(G, R)                                                                      \
+    launch_carved<-1>(select_kernel<G, PATHS, SPAN, R>, dim3(blocks), dim3(128), 0, stream, source, \
                  width, height, disparities, volume, uniqueness, disparity, keys, 1u)
-    if (g == 4) NXS_SELECT(4);
-    else if (g == 8) NXS_SELECT(8);
-    else NXS_SELECT(16);
+    if constexpr (PATHS == 3 || PATHS == 8) {
+        if (runs == 2 && g == 2) return NXS_SELECT(2, 2);
+    }
+    if constexpr (PATHS == 3) {
+        if (runs == 2) return NXS_SELECT(4, 2);
+        if (runs == 3) return g == 2 ? NXS_SELECT(2, 3) : NXS_SELECT(4, 3);
+        if (runs == 4) return NXS_SELECT(4, 4);
+    }
+    if (g == 4) NXS_SELECT(4, 1);
+    else if (g == 8) NXS_SELECT(8, 1);
+    else NXS_SELECT(16, 1);
 #undef NXS_SELECT
     return cudaGetLastError();
 }

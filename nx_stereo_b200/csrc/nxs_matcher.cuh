@@ -1065,79 +1065,87 @@ __host__ __device__ constexpr int select_position(int d) {
 // SPAN: the path volumes' disparity order (span_disparity).
 // PATHS 0: u16 sums in the volumes' order, not path volumes; -1: u16 sums in
 // the lane-split layout of sum_position (the summing path scan's output).
-template <int G, int PATHS, int SPAN = 0>
+// RUNS: runs of 16 disparities a lane takes (run member + G r is its r-th); above 1, the
+// lanes hold all D = 16 G RUNS disparities.
+template <int G, int PATHS, int SPAN = 0, int RUNS = 1>
 __device__ __forceinline__ void select_pixels(const void *__restrict__ source, int width,
                                               int height, int disparities, size_t volume,
                                               float uniqueness, float *__restrict__ disparity,
                                               uint32_t *__restrict__ keys,
                                               uint32_t *__restrict__ right_map, size_t block,
-                                              uint16_t (*values_of)[256], uint32_t one) {
+                                              uint16_t (*values_of)[RUNS == 1 ? 256 : 16 * G * RUNS],
+                                              uint32_t one) {
     constexpr int PIXELS = 128 / G;  // per 128 threads
     const int slot = (threadIdx.x % 128) / G, member = threadIdx.x % G;
     const size_t pixel = block * PIXELS + slot;
     const bool valid = pixel < (size_t)width * height;
     const int D = disparities;
-    const bool active = valid && member * 16 < D;
+    const bool active = valid && (RUNS > 1 || member * 16 < D);
     // A 32-bit remainder: pixel < 2^32, as 2^32 pixels' volumes (at least
     // 16 bytes a pixel) would not fit in device memory.
     const int x = valid ? (int)((uint32_t)pixel % (uint32_t)width) : 0;
-    const int d0 = member * 16;
-    uint32_t v[8];
+    uint32_t v[RUNS][8];
+    uint32_t best = 0xFFFFFFFFu;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = 0;
+    for (int run = 0; run < RUNS; ++run)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[run][k] = 0;
     if (active) {
-        const size_t at = pixel * D + d0;
-        if (PATHS <= 0) {
-            const uint16_t *base = static_cast<const uint16_t *>(source);
-            const uint4 *sums = reinterpret_cast<const uint4 *>(
-                PATHS == 0 ? base + at : base + pixel * D + 8 * member);
-            const uint4 a = __ldcg(sums);
-            const uint4 b = __ldcg(PATHS == 0 ? sums + 1 : sums + D / 16);
-            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-            v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-        } else {
-            const uint8_t *volumes = static_cast<const uint8_t *>(source) + at;
-            uint4 loaded[PATHS > 0 ? PATHS : 1];
 #pragma unroll
-            for (int p = 0; p < PATHS; ++p)  // every volume's load in flight at once
-                loaded[p] = __ldcs(reinterpret_cast<const uint4 *>(volumes + p * volume));
-            // The adds as multiply-adds by a run-time 1 (`one`), on the FMA pipe:
-            // the byte-wise pair sums carry nowhere (127 + 127 < 256), the u16
-            // sums neither (8 x 127 + 0x8000 < 0x10000).
+        for (int run = 0; run < RUNS; ++run) {
+            const int d0 = 16 * (member + G * run);
+            const size_t at = pixel * D + d0;
+            uint32_t(&w)[8] = v[run];
+            if (PATHS <= 0) {
+                const uint16_t *base = static_cast<const uint16_t *>(source);
+                const uint4 *sums = reinterpret_cast<const uint4 *>(
+                    PATHS == 0 ? base + at : base + pixel * D + 8 * member);
+                const uint4 a = __ldcg(sums);
+                const uint4 b = __ldcg(PATHS == 0 ? sums + 1 : sums + D / 16);
+                w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+                w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+            } else {
+                const uint8_t *volumes = static_cast<const uint8_t *>(source) + at;
+                uint4 loaded[PATHS > 0 ? PATHS : 1];
 #pragma unroll
-            for (int p = 0; p < PATHS; p += 2) {
-                const uint4 a = loaded[p];
-                uint4 both = a;
-                if (p + 1 < PATHS) {
-                    const uint4 b = loaded[p + 1];
-                    both = make_uint4(mad_lo(a.x, one, b.x), mad_lo(a.y, one, b.y),
-                                      mad_lo(a.z, one, b.z), mad_lo(a.w, one, b.w));
+                for (int p = 0; p < PATHS; ++p)  // every volume's load in flight at once
+                    loaded[p] = __ldcs(reinterpret_cast<const uint4 *>(volumes + p * volume));
+                // The adds as multiply-adds by a run-time 1 (`one`), on the FMA pipe:
+                // the byte-wise pair sums carry nowhere (127 + 127 < 256), the u16
+                // sums neither (8 x 127 + 0x8000 < 0x10000).
+#pragma unroll
+                for (int p = 0; p < PATHS; p += 2) {
+                    const uint4 a = loaded[p];
+                    uint4 both = a;
+                    if (p + 1 < PATHS) {
+                        const uint4 b = loaded[p + 1];
+                        both = make_uint4(mad_lo(a.x, one, b.x), mad_lo(a.y, one, b.y),
+                                          mad_lo(a.z, one, b.z), mad_lo(a.w, one, b.w));
+                    }
+                    uint32_t pair[8];
+                    unpack16(both, pair);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) w[k] = p == 0 ? pair[k] : mad_lo(pair[k], one, w[k]);
                 }
-                uint32_t pair[8];
-                unpack16(both, pair);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) v[k] = p == 0 ? pair[k] : mad_lo(pair[k], one, v[k]);
             }
-        }
-        if (x < d0 + 15) {  // disparities past the left edge lose
+            if (x < d0 + 15) {  // disparities past the left edge lose
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int lo = d0 + select_disparity<PATHS, SPAN>(2 * k);
+                    const int hi = d0 + select_disparity<PATHS, SPAN>(2 * k + 1);
+                    w[k] += (lo > x ? 0x8000u : 0u) | (hi > x ? 0x80000000u : 0u);
+                }
+            }
+            *reinterpret_cast<uint4 *>(&values_of[slot][d0]) = make_uint4(w[0], w[1], w[2], w[3]);
+            *reinterpret_cast<uint4 *>(&values_of[slot][d0 + 8]) =
+                make_uint4(w[4], w[5], w[6], w[7]);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                const int lo = d0 + select_disparity<PATHS, SPAN>(2 * k);
-                const int hi = d0 + select_disparity<PATHS, SPAN>(2 * k + 1);
-                v[k] += (lo > x ? 0x8000u : 0u) | (hi > x ? 0x80000000u : 0u);
+                const uint32_t lo = d0 + select_disparity<PATHS, SPAN>(2 * k);
+                const uint32_t hi = d0 + select_disparity<PATHS, SPAN>(2 * k + 1);
+                const uint32_t d = lo | (hi << 16);
+                best = min(best, min(__byte_perm(w[k], d, 0x1054), __byte_perm(w[k], d, 0x3276)));
             }
-        }
-        *reinterpret_cast<uint4 *>(&values_of[slot][d0]) = make_uint4(v[0], v[1], v[2], v[3]);
-        *reinterpret_cast<uint4 *>(&values_of[slot][d0 + 8]) = make_uint4(v[4], v[5], v[6], v[7]);
-    }
-    uint32_t best = 0xFFFFFFFFu;
-    if (active) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const uint32_t lo = d0 + select_disparity<PATHS, SPAN>(2 * k);
-            const uint32_t hi = d0 + select_disparity<PATHS, SPAN>(2 * k + 1);
-            const uint32_t d = lo | (hi << 16);
-            best = min(best, min(__byte_perm(v[k], d, 0x1054), __byte_perm(v[k], d, 0x3276)));
         }
     }
 #pragma unroll
@@ -1148,13 +1156,16 @@ __device__ __forceinline__ void select_pixels(const void *__restrict__ source, i
     uint32_t second = 0xFFFFFFFFu;
     if (active) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int lo = d0 + select_disparity<PATHS, SPAN>(2 * k);
-            const int hi = d0 + select_disparity<PATHS, SPAN>(2 * k + 1);
-            // d outside [winner - 1, winner + 1]
-            if ((unsigned)(lo - winner + 1) > 2u) second = min(second, v[k] & 0xFFFFu);
-            if ((unsigned)(hi - winner + 1) > 2u) second = min(second, v[k] >> 16);
-        }
+        for (int run = 0; run < RUNS; ++run)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int d0 = 16 * (member + G * run);
+                const int lo = d0 + select_disparity<PATHS, SPAN>(2 * k);
+                const int hi = d0 + select_disparity<PATHS, SPAN>(2 * k + 1);
+                // d outside [winner - 1, winner + 1]
+                if ((unsigned)(lo - winner + 1) > 2u) second = min(second, v[run][k] & 0xFFFFu);
+                if ((unsigned)(hi - winner + 1) > 2u) second = min(second, v[run][k] >> 16);
+            }
     }
 #pragma unroll
     for (int offset = G / 2; offset >= 1; offset /= 2)
