@@ -178,10 +178,11 @@ static bool encode_cost_maps(const uint8_t *costs, int width, int height, int di
 }
 
 // Whether the path scans take their full blocks' costs by tensor copies: 0
-// never, 2 always, 1 (the default) from kTilesFrom pixel-disparities on,
-// where they measured faster (1280x720x128: 295 against 300 us, 1920x1080x256:
-// 1329 against 1360 us); below it the per-lane copies were (728x544x128: 121
-// against 129 us, 364x272x64: 40 against 53 us). Results do not depend on it.
+// never, 2 always, 1 (the default) from kTilesFrom pixel-disparities on where the
+// sweep order (sweep_wanted) does not take the pair (1920x1080x256 1329 us against 1360
+// with per-lane copies, 1280x720x256 578 against 603 in the sweep). Below it the per-lane
+// copies were faster (728x544x128: 121 against 129 us, 364x272x64: 40 against 53 us).
+// Results do not depend on it.
 static std::atomic<int> g_path_tiles{1};
 constexpr size_t kTilesFrom = (size_t)96 << 20;
 void set_path_tiles(int mode) { g_path_tiles = mode < 0 || mode > 2 ? 1 : mode; }
@@ -189,6 +190,51 @@ int path_tiles() { return g_path_tiles; }
 static bool tiles_wanted(int width, int height, int disparities) {
     return g_path_tiles == 2 ||
            (g_path_tiles == 1 && (size_t)width * height * disparities >= kTilesFrom);
+}
+
+// The scan in the sweep order, one warp per block.
+template <int G, bool FULL>
+__global__ void __launch_bounds__(32)
+    paths_sweep_kernel(const uint8_t *__restrict__ costs, uint8_t *__restrict__ paths_out,
+                       const PathSetup s, bool down_first) {
+    __shared__ __align__(16) uint4 ring[kPrefetch * 32];
+    follow_previous_grid();
+    sweep_warp<G, FULL, kPrefetch>(costs, paths_out, s, down_first, blockIdx.x, threadIdx.x,
+                                   ring + threadIdx.x);
+}
+
+// Whether a pair's lines go in the sweep order: from 64 Mi pixel-disparities on (half the
+// L2), up to 128 disparities, where its warps of equal lines measured faster (us of the scan,
+// ranked lines or tiles -> sweep; 8 paths: 960x600x128 178 -> 163, 1024x768x96 214 -> 205,
+// 1024x768x128 252 -> 218, 1280x720x128 306 -> 277, 1600x1200x64 346 -> 286, 1600x900x128 465
+// -> 452, 1920x1080x128 695 -> 685; 3 paths: 1280x720x128 183 -> 171) and below it the ranked
+// ones, whose short lines fill the schedulers' gaps (1280x720x64 156 -> 170, 728x544x128 113
+// -> 119). With 16 lanes a line, two lines a warp make enough warps for the ranked lines and
+// the tile copies to balance, and the sweep is faster only at 192 disparities with 8 paths
+// from 160 Mi on (1280x720x192 491 -> 467, 1920x1080x192 1184 -> 1085; 800x600x192 233 -> 243),
+// at 256 with 3 paths (1280x720x256 283 -> 248), and with 8 by little from 256 to 768 Mi
+// (1280x720x256 578 -> 603, 1600x900x256 904 -> 900, 1920x1080x256 1333 -> 1321, 2560x1440x256
+// 2411 -> 2471): there the volume is read from memory once a direction in either order.
+constexpr size_t kMi = (size_t)1 << 20, kSweepFrom = 64 * kMi;
+static bool sweep_wanted(const PathSetup &s) {
+    if (g_path_tiles != 1 || s.volume < kSweepFrom) return false;
+    if (s.disparities <= 128) return true;
+    if (s.paths == 3) return s.disparities == 256;
+    return s.disparities == 256 ? s.volume >= 256 * kMi && s.volume < 768 * kMi
+                                : s.volume >= 160 * kMi;
+}
+
+// Warps a wave of the sweep holds (22 blocks a SM under the matcher's L1 split). In one wave
+// the rows, the longest lines, come first; in more the lines that go down do, so that they go
+// together (1920x1080x192 1172 -> 1085 us, 1280x720x128 277 and 278).
+constexpr int kSweepWave = 22 * 148;
+
+template <int G, bool FULL>
+static cudaError_t launch_sweep(const uint8_t *costs, uint8_t *paths_out, const PathSetup &s,
+                                cudaStream_t stream) {
+    const int warps = sweep_warps(s.width, s.height, s.paths, G);
+    return launch_after(paths_sweep_kernel<G, FULL>, dim3(warps), dim3(32), 0, stream, costs,
+                        paths_out, s, warps > kSweepWave);
 }
 
 unsigned path_wait_failures() {
@@ -271,6 +317,16 @@ static void launch_paths_in(const uint8_t *costs, uint8_t *paths_out, const Path
     const bool full = g * 2 * WORDS == s.disparities;
     CostMaps maps{};
     if constexpr (WORDS == 8 && PERMUTED) {
+        if (sweep_wanted(s)) {
+            if (g == 4) launch_sweep<4, true>(costs, paths_out, s, stream);
+            else if (g == 8)
+                full ? launch_sweep<8, true>(costs, paths_out, s, stream)
+                     : launch_sweep<8, false>(costs, paths_out, s, stream);
+            else
+                full ? launch_sweep<16, true>(costs, paths_out, s, stream)
+                     : launch_sweep<16, false>(costs, paths_out, s, stream);
+            return;
+        }
         if (full && tiles_wanted(s.width, s.height, s.disparities) &&
             encode_cost_maps(costs, s.width, s.height, s.disparities, &maps)) {
 #define NXS_TILED(G)                                                                           \

@@ -1022,6 +1022,114 @@ __device__ __forceinline__ void path_warp(const uint8_t *__restrict__ costs,
         costs, paths_out, s, p, line, own < s.lines[p], lane % G, ring, maps, tiles, bars);
 }
 
+// ---- the sweep order ----
+// The same lines for pairs whose cost volume does not stay in L2: every line of a direction
+// takes a step of the same image row at the same time. Columns do by themselves; a diagonal
+// line that leaves the image at one side goes on at the other, in the same row, as the line
+// that enters there (its costs from zero again), so a diagonal direction is W lines of H steps
+// instead of W + H - 1 of every length, and fills warps whose lines all have work to their
+// last step. The warps' order is the rows of both directions, then the three directions that
+// go down, column group by column group, then the three that go up; with down_first the rows
+// come after the lines that go down. Costs and path costs in span-16 order, 8 words a lane.
+__host__ __device__ inline int sweep_warps(int width, int height, int paths, int lanes) {
+    const int lines = 32 / lanes;
+    const int rows = (height + lines - 1) / lines, columns = (width + lines - 1) / lines;
+    return 2 * rows + (paths == 8 ? 6 : 1) * columns;
+}
+
+template <int G, bool FULL, int RING>
+__device__ __forceinline__ void sweep_warp(const uint8_t *__restrict__ costs,
+                                           uint8_t *__restrict__ paths_out, const PathSetup &s,
+                                           bool down_first, int warp, int lane, uint4 *ring) {
+    using Scan = LineScan<G, 8, FULL, 16, false>;
+    constexpr int LINES = 32 / G;
+    const int W = s.width, H = s.height, D = s.disparities, member = lane % G;
+    const int row_warps = 2 * ((H + LINES - 1) / LINES), column_warps = (W + LINES - 1) / LINES;
+    int p, group;
+    const int together = s.paths == 8 ? 3 : 1, down_warps = together * column_warps;
+    if (down_first && warp < down_warps + row_warps)
+        warp += warp < down_warps ? row_warps : -down_warps;
+    if (warp < row_warps) {
+        p = warp % 2;
+        group = warp / 2;
+    } else {
+        const int w = warp - row_warps;
+        const bool up = w >= down_warps;
+        const int k = up ? w - down_warps : w, which = k % together;
+        p = which == 0 ? (up ? 3 : 2) : (up ? 5 : 3) + which;  // 2, 4, 5 down, 3, 6, 7 up
+        group = k / together;
+    }
+    const int dy = s.dy[p], dx = s.dx[p];
+    // A group without a line of its own follows the last one without writing.
+    const int own = group * LINES + lane / G, last = dy == 0 ? H - 1 : W - 1;
+    const int line = min(own, last);
+    const int y0 = dy == 0 ? line : (dy > 0 ? 0 : H - 1);
+    const int x0 = dy == 0 ? (dx > 0 ? 0 : W - 1) : line;
+    const int steps = dy == 0 ? W : H;
+    const bool active = FULL || member * 16 < D, writes = own <= last && active;
+    const int stride = (dy * W + dx) * D, back = -dx * W * D;
+    // The step at which the line goes on at the other side, in the costs it asks for and in
+    // its own steps.
+    const int first_wrap = dy == 0 || dx == 0 ? 0x7FFFFFFF : (dx > 0 ? W - x0 : x0 + 1);
+    int wrap_ahead = first_wrap, wrap = first_wrap;
+    const size_t at = ((size_t)y0 * W + x0) * D + (active ? member * 16 : 0);
+    const uint8_t *ahead = costs + at;
+    uint8_t *dst = paths_out + (size_t)p * s.volume + at;
+
+    Scan scan;
+    scan.begin(s, member, active);
+    auto fetch = [&](int slot, bool valid) {
+        copy16_async(ring + slot * 32, valid ? ahead : costs, valid);
+        copy_commit();
+        ahead = advance(ahead, stride, s.one);
+    };
+    auto fetch_checked = [&](int slot, int step) {
+        if (step == wrap_ahead) {
+            ahead += back;
+            wrap_ahead += W;
+        }
+        fetch(slot, step < steps);
+    };
+#pragma unroll
+    for (int i = 0; i < RING - 1; ++i) fetch_checked(i, i);
+    for (int base = 0; base < steps; base += RING) {
+        // A block in which no line of the warp wraps, nor the costs it asks for, runs
+        // without the tests.
+        const bool plain = __all_sync(kFullMask, wrap >= base + RING &&
+                                                     wrap_ahead >= base + 2 * RING - 1) &&
+                           base + 2 * RING - 1 <= steps;
+        if (plain) {
+#pragma unroll
+            for (int i = 0; i < RING; ++i) {
+                fetch((i + RING - 1) % RING, true);
+                copy_wait<RING - 1>();
+                uint32_t cost[8];
+                scan.unpack(ring + i * 32, 32, cost);
+                scan.step(cost, dst, writes);
+                dst = advance(dst, stride, s.one);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < RING; ++i) {
+                const int step = base + i;
+                if (step >= steps) break;  // uniform across the warp
+                fetch_checked((i + RING - 1) % RING, step + RING - 1);
+                copy_wait<RING - 1>();
+                if (step == wrap) {
+                    scan.begin(s, member, active);
+                    dst += back;
+                    wrap += W;
+                }
+                uint32_t cost[8];
+                scan.unpack(ring + i * 32, 32, cost);
+                scan.step(cost, dst, writes);
+                dst = advance(dst, stride, s.one);
+            }
+        }
+    }
+    copy_wait<0>();
+}
+
 // Lanes per pixel (selection) or per line (paths with 16 disparities a lane),
 // 16 disparities each: a power of two.
 __host__ __device__ inline int group_lanes(int disparities) {
