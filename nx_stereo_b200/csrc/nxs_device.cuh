@@ -61,8 +61,9 @@ __device__ __forceinline__ void follow_previous_grid() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// CARVEOUT: the percentage of an SM's L1 memory a kernel asks for as shared memory (-1: the
-// driver's choice, by that kernel alone).
+// CARVEOUT: the percentage of an SM's L1 memory a kernel asks for as shared memory (-1, and
+// for blocks of more than 30 KB: the driver's choice, by that kernel alone).
+constexpr size_t kCarvedShared = 30 * 1024;
 template <int CARVEOUT, typename... Params, typename... Args>
 inline cudaError_t launch_carved(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared,
                                  cudaStream_t stream, Args &&...args) {
@@ -77,7 +78,7 @@ inline cudaError_t launch_carved(void (*kernel)(Params...), dim3 grid, dim3 bloc
     attribute[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
     attribute[1].val.sharedMemCarveout = (unsigned)CARVEOUT;
     config.attrs = attribute;
-    config.numAttrs = CARVEOUT < 0 ? 1 : 2;
+    config.numAttrs = CARVEOUT < 0 || shared > kCarvedShared ? 1 : 2;
     return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
 }
 
@@ -87,7 +88,9 @@ inline cudaError_t launch_carved(void (*kernel)(Params...), dim3 grid, dim3 bloc
 // out (four 1280x720x128 stream pairs 3,190 us, 2,951 with one split; 16 mixed pairs in a
 // batch 2,258 and 2,124). 60% (137 KB shared) holds 22 blocks of the path scan; the rest is
 // the room in which the selection's loads land: 40% and 100% measured 581 and 553 us for a
-// 1280x720x128 pair against 508.
+// 1280x720x128 pair against 508. Blocks of more than 30 KB are too few under it (census and
+// costs at 192 disparities, 31 KB, 94 us, 98 with the split; at 256, 41 KB, 272 and 281); at
+// 24 KB the line would shut the check of 1280 columns out (the stream pairs 2,784 -> 2,965).
 constexpr int kCarveout = 60;
 template <typename... Params, typename... Args>
 inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared,
