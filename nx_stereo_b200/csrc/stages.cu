@@ -222,7 +222,9 @@ __global__ void __launch_bounds__(kSpeckleX *kSpeckleY)
 // memory (2R + 1 values, into registers) serves every one of its pixels whose
 // window holds it: (kSpeckleRun + 2R) x (2R + 1) shared loads for
 // kSpeckleRun x ((2R + 1)^2 - 1) comparisons. The window's global loads are
-// all issued before any is stored.
+// all issued before any is stored. Values that support nothing (n <= 0, outside
+// the image) are staged as NaN, whose difference is within no max_diff, so a
+// comparison is the difference's alone (1280x720: 12.0 -> 11.6 us).
 constexpr int kSpeckleRun = 4;
 
 // The filtered values of this thread's kSpeckleRun pixels down column x from
@@ -250,7 +252,7 @@ __device__ __forceinline__ void despeckle_run(const float *__restrict__ disparit
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
         const int i = tid + k * THREADS;
-        if (i < TW * TH) window[i / TW][i % TW] = v[k];
+        if (i < TW * TH) window[i / TW][i % TW] = v[k] > 0.0f ? v[k] : __int_as_float(0x7FC00000);
     }
     __syncthreads();
     const int tx = threadIdx.x, top = threadIdx.y * kSpeckleRun;  // the run's first window row - R
@@ -274,7 +276,7 @@ __device__ __forceinline__ void despeckle_run(const float *__restrict__ disparit
             for (int dx = 0; dx <= 2 * R; ++dx) {
                 if (dy == R && dx == R) continue;
                 const float n = row[dx];
-                support[k] += (n > 0.0f) & (fabsf(fsub(n, centre[k])) <= max_diff);
+                support[k] += fabsf(fsub(n, centre[k])) <= max_diff;
             }
         }
     }
@@ -505,11 +507,12 @@ cudaError_t launch_despeckle_depth_cloud(const float *disparity, int width, int 
 // f64 and rounded to f32; then the columns' sums summed in f64 and rounded.
 //
 // A block takes kQualityX columns (a 32-byte sector of a row) with kQualityRows threads down
-// each: every thread sums every kQualityRows-th row of its column, so a column is 64 short
-// chains instead of one of H dependent steps, and 1280 columns are 160 blocks of 512 instead
-// of 10 of 128. The f64 partial sums are then added in a fixed order. The kernel also moves
+// each: every thread sums every kQualityRows-th row of its column, so a column is 128 short
+// chains instead of one of H dependent steps, and 1280 columns are 160 blocks of 1024 instead
+// of 10 of 128 (1280x720: 83 us, now 6.7; 8.5 with 64 threads a column). The f64 partial sums
+// are then added in a fixed order. The kernel also moves
 // the disparity into `previous`, both being in hand, which was a copy of its own.
-constexpr int kQualityX = 8, kQualityRows = 64, kQualityWarps = kQualityX * kQualityRows / 32;
+constexpr int kQualityX = 8, kQualityRows = 128, kQualityWarps = kQualityX * kQualityRows / 32;
 
 __global__ void __launch_bounds__(kQualityX *kQualityRows)
     quality_columns_kernel(const float *__restrict__ disparity, float *__restrict__ previous,

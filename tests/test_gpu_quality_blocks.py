@@ -1,4 +1,4 @@
-"""The quality sums at the edges of their kernel's blocks (8 columns, 64 rows in flight),
+"""The quality sums at the edges of their kernel's blocks (8 columns, 128 rows in flight),
 against the oracle. Sums of counts and values in f64, rounded to f32 once a column and once in
 all: whatever the order of the f64 additions, the two roundings bound the difference from the
 oracle's by 2^-23 + 2^-24 of the sum (all terms are positive), below 1e-6."""
@@ -18,7 +18,7 @@ def native():
     return n
 
 
-@pytest.mark.parametrize("w,h", [(1, 1), (7, 63), (8, 64), (9, 65), (33, 130), (500, 3)])
+@pytest.mark.parametrize("w,h", [(1, 1), (7, 63), (8, 64), (9, 65), (33, 130), (500, 3), (8, 128), (9, 257)])
 def test_quality_sums_at_the_edges_of_its_blocks(native, oracle, w, h):
     """Widths and heights around a block, a frame of unmatched pixels, and the disparity moved
     into `previous`."""
