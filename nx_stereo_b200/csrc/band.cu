@@ -13,11 +13,10 @@
 //   paths        u8  [P][H][W][B]   each direction's band path costs, <= p2 + 48
 //   selected f32 [H][W], keys u32 [H][W]; the check and median write the output.
 //
-// The band path scan keeps, per scan line, the previous pixel's path costs as
-// u16 values in a row of shared memory padded with +inf on both sides: moving
-// them to this pixel's band (by base - previous base) is a read of the row at
-// that offset, and candidates outside the previous band read +inf, which the
-// cap at the line's lowest cost + p2 makes the reference's p2.
+// The band path scan keeps, per scan line, the previous pixel's normalised
+// costs as u16 values in a row of shared memory padded with p2 on both sides:
+// moving them to this pixel's band (by base - previous base) is a read of the
+// row at that offset, and candidates outside the previous band read p2.
 #include <algorithm>
 #include <cstdio>
 
@@ -172,7 +171,7 @@ __global__ void __launch_bounds__(128)
 // with V candidates as V / 2 u16x2 words; a warp follows 32 / G lines.
 template <int BAND, int V>
 struct BandRow {
-    static constexpr int PAD = BAND + 4;             // u16 values of +inf each side
+    static constexpr int PAD = BAND + 4;             // u16 values of p2 each side
     static constexpr int ELEMENTS = BAND + 2 * PAD;  // of a line's row
     static constexpr int WORDS = ELEMENTS / 2;       // u32 words of a row
 };
@@ -189,10 +188,10 @@ __global__ void __launch_bounds__(32)
     const int lane = threadIdx.x, member = lane % G, slot_line = lane / G;
     uint32_t *row = rows[slot_line];
     const uint32_t p1x2 = (uint32_t)s.p1 * 0x10001u, p2x2 = (uint32_t)s.p2 * 0x10001u;
-    // pads of +inf, the band's middle zero (a line starts from zero)
+    // pads of p2, the band's middle zero (a line starts from zero)
     for (int w = member; w < Row::WORDS; w += G) {
         const int e = 2 * w;
-        row[w] = (e >= Row::PAD && e < Row::PAD + BAND) ? 0u : kInf2;
+        row[w] = (e >= Row::PAD && e < Row::PAD + BAND) ? 0u : p2x2;
     }
 
     // this warp's direction and line, as the full search assigns them
@@ -264,14 +263,8 @@ __global__ void __launch_bounds__(32)
         for (int k = 0; k < WORDS; ++k) {
             const uint32_t own = __byte_perm(even[k], even[k + 1], 0x5432);  // (window[2k+1], window[2k+2])
             const uint32_t neighbour = vmin2(even[k], even[k + 1]) + p1x2;
-            r[k] = __vimin3_u16x2(own, m2 + p2x2, neighbour) + cost[k] - m2;
+            r[k] = __vimin3_u16x2(own, p2x2, neighbour) + cost[k];
         }
-        // Into the row before the line's lowest cost is known: the next step takes it off,
-        // so the shuffles that find it run beside the row's way through shared memory
-        // instead of before it (728x544 band 16: a pair 176.5 -> 174.2 us).
-        __syncwarp();  // every lane has read the row
-#pragma unroll
-        for (int k = 0; k < WORDS; ++k) row[(Row::PAD + member * V) / 2 + k] = r[k];
         if (valid) {
             Chunk packed;
             uint32_t *words = reinterpret_cast<uint32_t *>(&packed);
@@ -279,12 +272,15 @@ __global__ void __launch_bounds__(32)
             for (int i = 0; i < V / 4; ++i) words[i] = __byte_perm(r[2 * i], r[2 * i + 1], 0x6420);
             *reinterpret_cast<Chunk *>(volume + pixel * BAND + member * V) = packed;
         }
-        // the line's lowest cost
+        // the line's lowest cost, then its normalised costs into the row
         uint32_t lowest = r[0];
 #pragma unroll
         for (int k = 1; k < WORDS; ++k) lowest = vmin2(lowest, r[k]);
         lowest = vmin2(lowest, __byte_perm(lowest, 0, 0x1032));
         m2 = line_minimum<G>(lowest);
+        __syncwarp();  // every lane has read the row
+#pragma unroll
+        for (int k = 0; k < WORDS; ++k) row[(Row::PAD + member * V) / 2 + k] = r[k] - m2;
         __syncwarp();
         previous_base = b;
         b = next_b;
