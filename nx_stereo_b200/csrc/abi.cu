@@ -1056,12 +1056,17 @@ extern "C" nxs_status nxs_quality_device(const float *d_disparity, float *d_prev
                                          uint32_t width, uint32_t height, float *d_sums,
                                          void *stream) {
     CHECK_SIZE(d_disparity && d_previous && d_sums && width > 0 && height > 0);
-    // The per-column sums live in a small stream-ordered allocation.
+    // The per-column sums live in a small stream-ordered allocation (a captured call's is the
+    // graph's own, whatever the pool, and no pool is made during a capture).
     float *columns = nullptr;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const cudaMemPool_t pool = small_pool();
-    if (!pool || cudaMallocFromPoolAsync(reinterpret_cast<void **>(&columns),
-                                         sizeof(float) * 5 * width, pool, s))
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capturing)) return NXS_CUDA_ERROR;
+    const bool captured = capturing != cudaStreamCaptureStatusNone;
+    const cudaMemPool_t pool = captured ? nullptr : small_pool();
+    const size_t bytes = sizeof(float) * 5 * width;
+    void **to = reinterpret_cast<void **>(&columns);
+    if (!pool ? cudaMallocAsync(to, bytes, s) : cudaMallocFromPoolAsync(to, bytes, pool, s))
         return NXS_CUDA_ERROR;
     cudaError_t e = launch_quality(d_disparity, d_previous, width, height, columns, d_sums, s);
     cudaFreeAsync(columns, s);

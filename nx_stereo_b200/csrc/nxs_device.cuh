@@ -29,7 +29,7 @@ __device__ __forceinline__ uint32_t vmin2(uint32_t a, uint32_t b) {
 // Per-halfword sum of two u16x2 words as f16x2 numbers on their bit patterns. Patterns
 // below 2048 are their value times 2^-24 (subnormals and the first normal binade), so
 // these adds are the integer adds below that; kInf16 is a NaN pattern, and a sum with
-// it is kInf16 again; kFar16 (8192.0) absorbs them. A two-operand FMA-pipe instruction:
+// it is kInf16 again; kFar2's 0x7000 (8192.0) absorbs them. A two-operand FMA-pipe instruction:
 // it issues beside the three-operand minimums of the integer pipe, which a multiply-add
 // does not (4 + 4 in 8.4 cycles a scheduler, against 13.2 with multiply-adds).
 __device__ __forceinline__ uint32_t add2(uint32_t a, uint32_t b) {

@@ -33,3 +33,26 @@ def test_quality_sums_at_the_edges_of_its_blocks(native, oracle, w, h):
                     g.ptr(d_sums), g.stream())
         assert np.allclose(g.host(d_sums), want, rtol=1e-6, atol=0)
         assert g.same_bits(g.host(d_previous), current)
+
+
+def test_a_captured_call_before_any_other():
+    """The first call of a process may be a captured one: its scratch is the graph's."""
+    import subprocess
+    import sys
+
+    code = """
+import numpy as np, torch
+from nx_stereo_b200 import native
+d = torch.rand((40, 50), device="cuda") * 50
+previous, sums = torch.full_like(d, -1.0), torch.empty(5, device="cuda")
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    native.call("nxs_quality_device", d.data_ptr(), previous.data_ptr(), 50, 40,
+                sums.data_ptr(), torch.cuda.current_stream().cuda_stream)
+graph.replay()
+torch.cuda.synchronize()
+assert sums[0].item() == 2000 and abs(sums[1].item() / d.sum().item() - 1) < 1e-5
+assert torch.equal(previous, d)
+"""
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
