@@ -463,11 +463,17 @@ __global__ void __launch_bounds__(128)
                                   disparity, keys, nullptr, blockIdx.x, values_of, one);
 }
 
-// select_kernel with a grid of `resident` blocks that step through the
+// select_kernel with a grid of a few resident blocks a SM that step through the
 // pixel blocks: a selection run beside another stream's path scan holds
-// fewer warps a SM while it streams the path volumes.
+// fewer warps a SM while it streams the path volumes. Held to the registers that
+// the default grid's blocks find on an SM: without the bound the compiler overlaps
+// two pixel blocks and takes 128 to 167 registers for 3 and 4 runs a lane, so that
+// an SM holds 3 or 4 blocks, which take the path scan's room besides (stream-engine
+// batches of 8 mixed sizes with 3 paths: 96 disparities 951 -> 904 us, 192 1,630 ->
+// 1,536, 256 2,123 -> 1,849).
+constexpr int kLeanBlocks = 8;
 template <int G, int PATHS, int SPAN, int RUNS>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, kLeanBlocks)
     select_lean_kernel(const void *__restrict__ source, int width, int height, int disparities,
                        size_t volume, float uniqueness, float *__restrict__ disparity,
                        uint32_t *__restrict__ keys, uint32_t one, size_t blocks) {
@@ -484,7 +490,7 @@ __global__ void __launch_bounds__(128)
 // (0: one block for each pixel block). 8 measured best end to end on the
 // 728x544x128 chain: 2% above the full grid, 16 (above the 12 that fit a SM at
 // 39 registers) 7% below it.
-static std::atomic<int> g_lean_select{8};
+static std::atomic<int> g_lean_select{kLeanBlocks};
 void set_lean_select(int blocks_per_sm) { g_lean_select = blocks_per_sm < 0 ? 0 : blocks_per_sm; }
 int lean_select() { return g_lean_select.load(); }
 
