@@ -465,15 +465,15 @@ __global__ void __launch_bounds__(128)
 
 // select_kernel with a grid of a few resident blocks a SM that step through the
 // pixel blocks: a selection run beside another stream's path scan holds
-// fewer warps a SM while it streams the path volumes. Held to the registers that
-// the default grid's blocks find on an SM: without the bound the compiler overlaps
-// two pixel blocks and takes 128 to 167 registers for 3 and 4 runs a lane, so that
-// an SM holds 3 or 4 blocks, which take the path scan's room besides (stream-engine
-// batches of 8 mixed sizes with 3 paths: 96 disparities 951 -> 904 us, 192 1,630 ->
-// 1,536, 256 2,123 -> 1,849).
+// fewer warps a SM while it streams the path volumes. With more than one run a lane
+// held to the registers that the default grid's blocks find on an SM: without the
+// bound the compiler takes 128 and 167 for 3 and 4 runs, so that an SM holds 4 or 3
+// blocks, which take the path scan's room besides (stream-engine batches of 8 mixed
+// sizes with 3 paths: 96 disparities 924 -> 877 us, 192 1,565 -> 1,477, 256 1,919 ->
+// 1,837). One run a lane takes 39 to 47 by itself, and 53 under the bound.
 constexpr int kLeanBlocks = 8;
 template <int G, int PATHS, int SPAN, int RUNS>
-__global__ void __launch_bounds__(128, kLeanBlocks)
+__global__ void __launch_bounds__(128, RUNS > 1 ? kLeanBlocks : 0)
     select_lean_kernel(const void *__restrict__ source, int width, int height, int disparities,
                        size_t volume, float uniqueness, float *__restrict__ disparity,
                        uint32_t *__restrict__ keys, uint32_t one, size_t blocks) {
