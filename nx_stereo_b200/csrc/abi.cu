@@ -1759,7 +1759,7 @@ extern "C" nxs_status nxs_run_async(nxs_context *c, uint32_t id, uint32_t n_memb
             e = cudaStreamWaitEvent(s, seg->freed[lane], 0);
             if (!e)
                 e = run_matcher_front(slot.images[0], slot.images[1], g.width, g.height,
-                                      m.disparities, m.paths, l.sgm.p1, l.sgm.p2, ms, s);
+                                      m.disparities, m.paths, l.sgm.p1, l.sgm.p2, ms, s, true);
             if (!e) e = cudaEventRecord(seg->carved[lane], s);
             if (!e) e = cudaStreamWaitEvent(back, seg->carved[lane], 0);
             if (!e)

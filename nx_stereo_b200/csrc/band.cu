@@ -358,17 +358,20 @@ __global__ void __launch_bounds__(128)
 }
 
 // ---------------------------------------------------------------- launchers
+// The band kernels leave the L1's split to the driver: a pair runs them alone, and pairs of
+// several streams at once measured no slower than before the other kernels shared a split
+// (two 728x544 pairs 342 -> 278 us, 1280x720 at band 32 1,082 -> 1,067).
 cudaError_t launch_shrink_pair(const uint8_t *left, const uint8_t *right, int width, int height,
                                uint8_t *left_half, uint8_t *right_half, cudaStream_t stream) {
     const int n = (width / 2) * (height / 2);
-    return launch_carved<-1>(shrink_pair_kernel, dim3((n + 255) / 256), dim3(256), 0, stream, left,
+    return launch_alone(shrink_pair_kernel, dim3((n + 255) / 256), dim3(256), 0, stream, left,
                         right, width, height, left_half, right_half);
 }
 
 cudaError_t launch_band_base(const float *coarse, int coarse_width, int coarse_height, int band,
                              int margin, int32_t *base, cudaStream_t stream) {
     const int n = coarse_width * coarse_height;
-    return launch_carved<-1>(band_base_kernel, dim3((n + 255) / 256), dim3(256), 0, stream, coarse,
+    return launch_alone(band_base_kernel, dim3((n + 255) / 256), dim3(256), 0, stream, coarse,
                         coarse_width, coarse_height, band, margin, base);
 }
 
@@ -378,10 +381,10 @@ cudaError_t launch_census_window(const uint8_t *left, const uint8_t *right, int 
     if (window == 0)
         return launch_census(left, right, width, height, left_codes, right_codes, stream);
     const dim3 grid((width + 127) / 128, height, 2);
-    return window == 2 ? launch_carved<-1>(census_dense_kernel<true>, grid, dim3(128), 0, stream, left,
+    return window == 2 ? launch_alone(census_dense_kernel<true>, grid, dim3(128), 0, stream, left,
                                       right, width, height, left_codes, right_codes)
-                       : launch_carved<-1>(census_dense_kernel<false>, grid, dim3(128), 0, stream,
-                                      left, right, width, height, left_codes, right_codes);
+                       : launch_alone(census_dense_kernel<false>, grid, dim3(128), 0, stream, left,
+                                      right, width, height, left_codes, right_codes);
 }
 
 cudaError_t launch_band_costs(const uint64_t *left_codes, const uint64_t *right_codes,
@@ -389,7 +392,7 @@ cudaError_t launch_band_costs(const uint64_t *left_codes, const uint64_t *right_
                               uint8_t *costs, cudaStream_t stream) {
     const dim3 grid((width + 127) / 128, height);
 #define NXS_BAND_COSTS(B)                                                                      \
-    launch_carved<-1>(band_costs_kernel<B>, grid, dim3(128), 0, stream, left_codes, right_codes,   \
+    launch_alone(band_costs_kernel<B>, grid, dim3(128), 0, stream, left_codes, right_codes,     \
                  base, width, height, costs)
     switch (band) {
     case 8: return NXS_BAND_COSTS(8);
@@ -411,7 +414,7 @@ cudaError_t launch_band_paths(const uint8_t *costs, const int32_t *base, int wid
     PathSetup s;
     const int total = path_setup(width, height, band, paths, p1, p2, band / v, &s);
 #define NXS_BAND_PATHS(B, VV)                                                                  \
-    launch_carved<-1>(band_paths_kernel<B, VV>, dim3(total), dim3(32), 0, stream, costs, base, out, s)
+    launch_alone(band_paths_kernel<B, VV>, dim3(total), dim3(32), 0, stream, costs, base, out, s)
     switch (band) {
     case 8: return NXS_BAND_PATHS(8, 4);
     case 16: return NXS_BAND_PATHS(16, 4);
@@ -428,7 +431,7 @@ cudaError_t launch_band_select(const uint8_t *paths_in, const int32_t *base, int
     const size_t pixels = (size_t)width * height, volume = pixels * band;
     const dim3 grid((unsigned)((pixels + 127) / 128));
 #define NXS_BAND_SELECT(B, P)                                                                  \
-    launch_carved<-1>(band_select_kernel<B, P>, grid, dim3(128), 0, stream, paths_in, base, width,   \
+    launch_alone(band_select_kernel<B, P>, grid, dim3(128), 0, stream, paths_in, base, width,   \
                  height, disparities, volume, uniqueness, disparity, keys)
 #define NXS_BAND_SELECT_PATHS(B) return paths == 8 ? NXS_BAND_SELECT(B, 8) : NXS_BAND_SELECT(B, 3)
     switch (band) {

@@ -64,8 +64,9 @@ cudaError_t launch_costs(const uint64_t *left_codes, const uint64_t *right_codes
                          int span) {
     dim3 grid((width + kCostPixels - 1) / kCostPixels, height);
     const size_t shared = costs_shared_bytes(disparities);
+    // By its entry point alone, with the driver's split (1280x720x240: 118.3 us, 119.4 in ours).
 #define NXS_COSTS(S)                                                                          \
-    launch_after(costs_kernel<S>, grid, dim3(128), shared, stream, left_codes, right_codes,   \
+    launch_alone(costs_kernel<S>, grid, dim3(128), shared, stream, left_codes, right_codes,   \
                  width, disparities, costs)
     if (span == 16) NXS_COSTS(16);
     else if (span == 8) NXS_COSTS(8);
@@ -89,13 +90,20 @@ __global__ void __launch_bounds__(128)
 }
 
 cudaError_t launch_census_costs(const uint8_t *left, const uint8_t *right, int width, int height,
-                                int disparities, uint8_t *costs, cudaStream_t stream, int span) {
+                                int disparities, uint8_t *costs, cudaStream_t stream, int span,
+                                bool beside) {
     if (disparities < 16 || disparities > 256 || disparities % 16) return cudaErrorInvalidValue;
     dim3 grid((width + kCensusCostPixels - 1) / kCensusCostPixels, height);
     const size_t shared = census_costs_shared_bytes(kCensusCostPixels, disparities);
+    // By itself in the matcher's split up to 128 disparities, where an SM holds 7 of its blocks
+    // or more there and the split costs nothing; from 144 on they are too few (1280x720: 144
+    // 77.1 us, 79.2 in the split; 176 87.8 and 92.7; 192 93.6 and 98). Beside other pairs
+    // always: out of it the kernel shuts their selections out (six 1280x720 pairs of a segment
+    // with 3 paths at 192 disparities 4,390 us, 3,210 in the split; at 256 5,550 and 3,920).
+    const int split = beside || disparities <= 128 ? kCarveout : kDriversSplit;
 #define NXS_CENSUS_COSTS(S)                                                                   \
-    launch_after(census_costs_kernel<S>, grid, dim3(128), shared, stream, left, right, width, \
-                 height, disparities, costs)
+    launch_with(split, census_costs_kernel<S>, grid, dim3(128), shared, stream, left, right,  \
+                width, height, disparities, costs)
     if (span == 16) NXS_CENSUS_COSTS(16);
     else if (span == 8) NXS_CENSUS_COSTS(8);
     else NXS_CENSUS_COSTS(0);
@@ -329,8 +337,9 @@ static void launch_paths_in(const uint8_t *costs, uint8_t *paths_out, const Path
         }
         if (full && tiles_wanted(s.width, s.height, s.disparities) &&
             encode_cost_maps(costs, s.width, s.height, s.disparities, &maps)) {
+            // 16 KB of tiles a block: too few of them in the matcher's split.
 #define NXS_TILED(G)                                                                           \
-    launch_carved<-1>(paths_kernel<G, 8, true, 16, false, true>, dim3(total), dim3(32), 0, stream, \
+    launch_alone(paths_kernel<G, 8, true, 16, false, true>, dim3(total), dim3(32), 0, stream, \
                  costs, paths_out, s, maps)
             if (g == 4) NXS_TILED(4);
             else if (g == 8) NXS_TILED(8);
@@ -545,9 +554,10 @@ static cudaError_t launch_select(const void *source, int width, int height, int 
 #undef NXS_LEAN
         return cudaGetLastError();
     }
+    // The whole grid at once wants the cache that a small split leaves its loads.
 #define NXS_SELECT(G, R)                                                                      \
-    launch_carved<-1>(select_kernel<G, PATHS, SPAN, R>, dim3(blocks), dim3(128), 0, stream, source, \
-                 width, height, disparities, volume, uniqueness, disparity, keys, 1u)
+    launch_alone(select_kernel<G, PATHS, SPAN, R>, dim3(blocks), dim3(128), 0, stream,        \
+                 source, width, height, disparities, volume, uniqueness, disparity, keys, 1u)
     if constexpr (PATHS == 3 || PATHS == 8) {
         if (runs == 2 && g == 2) return NXS_SELECT(2, 2);
     }
@@ -724,9 +734,11 @@ static cudaError_t allow_check_median_shared() {
     return e;
 }
 
+constexpr int kWideCheckCarveout = 80;
+
 cudaError_t launch_check_median(const float *disparity, const uint32_t *keys, int width,
                                 int height, int stage_mask, float *filtered,
-                                cudaStream_t stream) {
+                                cudaStream_t stream, bool beside) {
     const size_t shared = check_median_shared_bytes(width);
     // Wide images need more than the default 48 KB: allowed once per device
     // (the attribute belongs to the device current when it is set), for the widest.
@@ -734,9 +746,20 @@ cudaError_t launch_check_median(const float *disparity, const uint32_t *keys, in
         const cudaError_t allowed = allow_check_median_shared();
         if (allowed != cudaSuccess) return allowed;
     }
-    return launch_after(check_median_kernel, dim3((height + kBandRows - 1) / kBandRows),
-                        dim3(256), shared, stream, disparity, keys, width, height, stage_mask,
-                        filtered);
+    // By itself in the matcher's split while its blocks run in one wave there too (1281x720: 5
+    // a SM, 12.1 us in either; 1360x768, 4 a SM, 14.6 and 15.4 in the split; 1920x1080 26.1 and
+    // 28.7). Beside other pairs never in the driver's choice, which for these blocks is the
+    // largest split and shuts the other kernels out (four pairs of a stream, driver's choice
+    // and the matcher's split: 1360x768x64 2,310 and 1,960 us, 1440x810x64 2,940 and 2,230,
+    // 1680x945x128 5,230 and 4,530), but from 1500 columns in the next one, of 196 KB (at 80%):
+    // 1600x900x128 4,127 -> 4,005, 1520x855x128 3,691 -> 3,637; 1440x810x64 2,211 -> 2,266 and
+    // 1360x768x64 1,955 -> 2,597.
+    const int blocks = (height + kBandRows - 1) / kBandRows;
+    int split = kDriversSplit;
+    if (beside) split = width >= 1500 ? kWideCheckCarveout : kCarveout;
+    else if ((size_t)blocks <= kSplitBytes / (shared + kBlockReserve) * kSMs) split = kCarveout;
+    return launch_with(split, check_median_kernel, dim3(blocks), dim3(256), shared, stream,
+                       disparity, keys, width, height, stage_mask, filtered);
 }
 
 // ---------------------------------------------------------------- the matcher
@@ -763,12 +786,13 @@ MatcherScratch carve_matcher_scratch(void *base, int width, int height, int disp
 
 cudaError_t run_matcher_front(const uint8_t *left, const uint8_t *right, int width, int height,
                               int disparities, int paths, int p1, int p2,
-                              const MatcherScratch &s, cudaStream_t stream) {
+                              const MatcherScratch &s, cudaStream_t stream, bool beside) {
     cudaError_t e;
     // The intermediates are in the permuted order of the path lanes' span
     // (span_disparity).
     const int span = matcher_span(disparities);
-    if ((e = launch_census_costs(left, right, width, height, disparities, s.costs, stream, span)))
+    if ((e = launch_census_costs(left, right, width, height, disparities, s.costs, stream, span,
+                                 beside)))
         return e;
     if (path_sums_wanted(width, height, disparities))  // the aggregate in the path volumes' room
         return launch_paths_sums(s.costs, width, height, disparities, paths, p1, p2,
@@ -789,7 +813,8 @@ cudaError_t run_matcher_back(int width, int height, int disparities, int paths,
                                 s.selected, s.keys, stream, matcher_span(disparities),
                                 beside ? g_lean_select.load() : 0);
     if (e) return e;
-    return launch_check_median(s.selected, s.keys, width, height, stage_mask, disparity, stream);
+    return launch_check_median(s.selected, s.keys, width, height, stage_mask, disparity, stream,
+                               beside);
 }
 
 cudaError_t run_matcher(const uint8_t *left, const uint8_t *right, int width, int height,
@@ -797,7 +822,8 @@ cudaError_t run_matcher(const uint8_t *left, const uint8_t *right, int width, in
                         int stage_mask, const MatcherScratch &s, float *disparity,
                         cudaStream_t stream, bool beside) {
     const cudaError_t e =
-        run_matcher_front(left, right, width, height, disparities, paths, p1, p2, s, stream);
+        run_matcher_front(left, right, width, height, disparities, paths, p1, p2, s, stream,
+                          beside);
     if (e) return e;
     return run_matcher_back(width, height, disparities, paths, uniqueness, stage_mask, s,
                             disparity, stream, beside);

@@ -61,12 +61,21 @@ __device__ __forceinline__ void follow_previous_grid() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// CARVEOUT: the percentage of an SM's L1 memory a kernel asks for as shared memory (-1, and
-// for blocks of more than 30 KB: the driver's choice, by that kernel alone).
-constexpr size_t kCarvedShared = 30 * 1024;
-template <int CARVEOUT, typename... Params, typename... Args>
-inline cudaError_t launch_carved(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared,
-                                 cudaStream_t stream, Args &&...args) {
+// The kernels that run beside one another (a segment's two lanes, a batch's streams) ask
+// for the same split of the L1 between shared memory and cache: an SM that holds blocks of
+// one split takes none of another, so with the driver's choice for each kernel a path scan
+// and a selection shut each other out (four 1280x720x128 stream pairs 3,190 us, 2,951 with
+// one split; 16 mixed pairs in a batch 2,258 and 2,124). 60% gives the 164 KB split, which
+// holds 23 blocks of the path scan (6 KB and the 1 KB an SM reserves for each) and the 32 it
+// takes at most of the sweep's; the rest is the room in which the selection's loads land: 40%
+// and 100% measured 581 and 553 us for a 1280x720x128 pair against 508. A kernel whose blocks
+// are too few there by itself, or that runs by itself, leaves the choice to the driver
+// (launch_alone), each for the reason given at its launch.
+constexpr int kCarveout = 60, kDriversSplit = 0, kSMs = 148;
+constexpr size_t kSplitBytes = 164 * 1024, kBlockReserve = 1024;
+template <typename... Params, typename... Args>
+inline cudaError_t launch_with(int carveout, void (*kernel)(Params...), dim3 grid, dim3 block,
+                               size_t shared, cudaStream_t stream, Args &&...args) {
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
     config.blockDim = block;
@@ -76,27 +85,24 @@ inline cudaError_t launch_carved(void (*kernel)(Params...), dim3 grid, dim3 bloc
     attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attribute[0].val.programmaticStreamSerializationAllowed = 1;
     attribute[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-    attribute[1].val.sharedMemCarveout = (unsigned)CARVEOUT;
+    attribute[1].val.sharedMemCarveout = (unsigned)carveout;
     config.attrs = attribute;
-    config.numAttrs = CARVEOUT < 0 || shared > kCarvedShared ? 1 : 2;
+    config.numAttrs = carveout == kDriversSplit ? 1 : 2;
     return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
 }
 
-// The kernels that run beside one another (a segment's two lanes, a batch's streams) ask
-// for the same split of the L1: an SM that holds blocks of one split takes none of another,
-// so with the driver's choice for each kernel a path scan and a selection shut each other
-// out (four 1280x720x128 stream pairs 3,190 us, 2,951 with one split; 16 mixed pairs in a
-// batch 2,258 and 2,124). 60% (137 KB shared) holds 22 blocks of the path scan; the rest is
-// the room in which the selection's loads land: 40% and 100% measured 581 and 553 us for a
-// 1280x720x128 pair against 508. Blocks of more than 30 KB are too few under it (census and
-// costs at 192 disparities, 31 KB, 94 us, 98 with the split; at 256, 41 KB, 272 and 281); at
-// 24 KB the line would shut the check of 1280 columns out (the stream pairs 2,784 -> 2,965).
-constexpr int kCarveout = 60;
 template <typename... Params, typename... Args>
 inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared,
                                 cudaStream_t stream, Args &&...args) {
-    return launch_carved<kCarveout>(kernel, grid, block, shared, stream,
-                                    std::forward<Args>(args)...);
+    return launch_with(kCarveout, kernel, grid, block, shared, stream,
+                       std::forward<Args>(args)...);
+}
+
+template <typename... Params, typename... Args>
+inline cudaError_t launch_alone(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared,
+                                cudaStream_t stream, Args &&...args) {
+    return launch_with(kDriversSplit, kernel, grid, block, shared, stream,
+                       std::forward<Args>(args)...);
 }
 
 }  // namespace nxs

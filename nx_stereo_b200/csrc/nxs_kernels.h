@@ -32,10 +32,11 @@ cudaError_t launch_costs(const uint64_t *left_codes, const uint64_t *right_codes
                          int height, int disparities, uint8_t *costs, cudaStream_t stream,
                          int span = 0);
 // The census of both images and the costs in one launch (the codes stay in
-// shared memory): the same costs as launch_census then launch_costs.
+// shared memory): the same costs as launch_census then launch_costs. beside: as
+// in run_matcher.
 cudaError_t launch_census_costs(const uint8_t *left, const uint8_t *right, int width, int height,
                                 int disparities, uint8_t *costs, cudaStream_t stream,
-                                int span = 0);
+                                int span = 0, bool beside = false);
 // paths_out[p][y][x][d] (u8) for p < paths; span 8 or 16: costs and path
 // costs in that permuted order (span 0: natural).
 cudaError_t launch_paths(const uint8_t *costs, int width, int height, int disparities, int paths,
@@ -79,9 +80,11 @@ cudaError_t launch_select_sums(const uint16_t *sums, int width, int height, int 
                                cudaStream_t stream);
 cudaError_t launch_consistency(const float *disparity, const uint32_t *keys, int width,
                                int height, float *checked, cudaStream_t stream);
-// The left-right check and the median (with the stage mask) in one pass.
+// The left-right check and the median (with the stage mask) in one pass. beside:
+// as in run_matcher.
 cudaError_t launch_check_median(const float *disparity, const uint32_t *keys, int width,
-                                int height, int stage_mask, float *filtered, cudaStream_t stream);
+                                int height, int stage_mask, float *filtered, cudaStream_t stream,
+                                bool beside = false);
 cudaError_t launch_median3(const float *image, int width, int height, int stage_mask,
                            float *filtered, cudaStream_t stream);
 
@@ -141,8 +144,8 @@ MatcherScratch carve_matcher_scratch(void *base, int width, int height, int disp
 
 // The whole matcher on device buffers: census, costs, paths, selection, the
 // check and the median (with Stage.Disparity's mask when stage_mask). beside:
-// the selection runs beside other pairs' path scans (the lean grid of
-// set_lean_select).
+// the pair's kernels run beside other pairs' (the selection as the lean grid of
+// set_lean_select, and all of them in one split of the L1).
 cudaError_t run_matcher(const uint8_t *left, const uint8_t *right, int width, int height,
                         int disparities, int paths, int p1, int p2, float uniqueness,
                         int stage_mask, const MatcherScratch &scratch, float *disparity,
@@ -152,7 +155,8 @@ cudaError_t run_matcher(const uint8_t *left, const uint8_t *right, int width, in
 // one stream; a segment may run them on two, pairs apart.
 cudaError_t run_matcher_front(const uint8_t *left, const uint8_t *right, int width, int height,
                               int disparities, int paths, int p1, int p2,
-                              const MatcherScratch &scratch, cudaStream_t stream);
+                              const MatcherScratch &scratch, cudaStream_t stream,
+                              bool beside = false);
 cudaError_t run_matcher_back(int width, int height, int disparities, int paths,
                              float uniqueness, int stage_mask, const MatcherScratch &scratch,
                              float *disparity, cudaStream_t stream, bool beside = false);
