@@ -508,14 +508,11 @@ int lean_select() { return g_lean_select.load(); }
 // too few to hide that, and with 96 or 192 disparities a quarter of the lanes idle. More
 // runs a lane measured (us, one run -> this table): 3 paths 1280x720x64 52.9 -> 39.4, x128
 // 87.3 -> 72.0, x256 174.8 -> 134.5 (two runs 146.1), 641x479x96 30.1 -> 18.0, 1277x713x192
-// 171.0 -> 104.2; 8 paths 1280x720x64 92.8 -> 79.7. With 8 paths that is so only at 64
-// disparities and above half a million pixels: the smaller frames stay in L2 and want the
-// warps (364x272x64 within a coarse-to-fine pair 176.5 us, 178.4 with two runs; a lean grid
-// in a batch 2,119 and 2,150), and with more disparities the volumes' bytes bound it, which
-// fewer lanes a pixel read in smaller pieces (728x544x128 61.7, 69.3 with two runs;
+// 171.0 -> 104.2. With 8 paths the volumes' bytes bound it, which fewer lanes a pixel read in
+// smaller pieces: within a pair one run is faster at every size (860x640x64 56.9, 64.8 with
+// two runs; 1280x720x64 91.7 and 97.5; 1600x900x64 141 and 159; 728x544x128 61.7 and 69.3;
 // 641x479x96 44.8, 77.4 with three).
-static int select_runs(int disparities, int paths, size_t pixels, bool lean) {
-    if (paths == 8) return disparities == 64 && !lean && pixels >= ((size_t)1 << 19) ? 2 : 1;
+static int select_runs(int disparities, int paths) {
     if (paths != 3) return 1;
     switch (disparities) {
     case 64: case 128: return 2;
@@ -531,7 +528,7 @@ static cudaError_t launch_select(const void *source, int width, int height, int 
                                  cudaStream_t stream, int lean = 0) {
     const size_t pixels = (size_t)width * height;
     const size_t volume = pixels * disparities;
-    const int runs = select_runs(disparities, PATHS, pixels, lean > 0);
+    const int runs = select_runs(disparities, PATHS);
     const int g = runs == 1 ? group_lanes(disparities) : disparities / (16 * runs);
     const unsigned blocks = (unsigned)((pixels + 128 / g - 1) / (128 / g));
     if (lean > 0) {
@@ -558,11 +555,8 @@ static cudaError_t launch_select(const void *source, int width, int height, int 
 #define NXS_SELECT(G, R)                                                                      \
     launch_alone(select_kernel<G, PATHS, SPAN, R>, dim3(blocks), dim3(128), 0, stream,        \
                  source, width, height, disparities, volume, uniqueness, disparity, keys, 1u)
-    if constexpr (PATHS == 3 || PATHS == 8) {
-        if (runs == 2 && g == 2) return NXS_SELECT(2, 2);
-    }
     if constexpr (PATHS == 3) {
-        if (runs == 2) return NXS_SELECT(4, 2);
+        if (runs == 2) return g == 2 ? NXS_SELECT(2, 2) : NXS_SELECT(4, 2);
         if (runs == 3) return g == 2 ? NXS_SELECT(2, 3) : NXS_SELECT(4, 3);
         if (runs == 4) return NXS_SELECT(4, 4);
     }
