@@ -214,9 +214,11 @@ uint32_t nxs_path_sums(uint32_t width, uint32_t height, uint32_t disparities);
  * steps that every line of a warp covers come as bulk tensor copies, one
  * [8][D] tile a line, into shared memory; without, every lane copies its own
  * 16 bytes a step. Mode 0 never tiles, 2 always, 1 (the default) as each
- * size measured fastest: tiles from 96 Mi pixel-disparities a pair on, but
- * where the lines go in the sweep order (every line of a direction at the same
- * image row), which only mode 1 takes, from 64 Mi on at most disparity counts.
+ * size measured fastest: tiles from 96 Mi pixel-disparities a pair on with 8
+ * paths, from 560 Mi with 3, but where the lines go in the sweep order (every
+ * line of a direction at the same image row), which only mode 1 takes, in a
+ * range of sizes for each disparity and path count (from 64 Mi on at the
+ * earliest; 8 paths at 256 and 3 at 64 and 192 disparities never).
  * A tuning knob for the whole library; results do not depend on it.
  * nxs_path_wait_failures: the path scans' waits on those copies that gave up
  * on the current device (each wait is bounded, about 1 s; 0 unless a copy

@@ -186,18 +186,20 @@ static bool encode_cost_maps(const uint8_t *costs, int width, int height, int di
 }
 
 // Whether the path scans take their full blocks' costs by tensor copies: 0
-// never, 2 always, 1 (the default) from kTilesFrom pixel-disparities on where the
-// sweep order (sweep_wanted) does not take the pair (1920x1080x256 1329 us against 1360
-// with per-lane copies, 1280x720x256 578 against 603 in the sweep). Below it the per-lane
-// copies were faster (728x544x128: 121 against 129 us, 364x272x64: 40 against 53 us).
+// never, 2 always, 1 (the default) as measured (us of the scan, per-lane copies of the
+// ranked lines -> tiles) where the sweep order (sweep_wanted) does not take the pair: with
+// 8 paths from 96 Mi pixel-disparities on (1920x1080x256 1375 -> 1332, 1920x1080x128 750 ->
+// 680, 3600x2000x64 1561 -> 1305; 728x544x128 121 -> 129, 364x272x64 40 -> 53), with 3, whose
+// lines alone fill the warps, from 560 Mi on (3840x2600x64 835 -> 768, 3840x2160x128 1276 ->
+// 1163; 3840x2160x64, 506 Mi, 569 -> 604, 1920x1080x128 278 -> 300, 900x600x256 140 -> 154).
 // Results do not depend on it.
 static std::atomic<int> g_path_tiles{1};
-constexpr size_t kTilesFrom = (size_t)96 << 20;
+constexpr size_t kMi = (size_t)1 << 20;
 void set_path_tiles(int mode) { g_path_tiles = mode < 0 || mode > 2 ? 1 : mode; }
 int path_tiles() { return g_path_tiles; }
-static bool tiles_wanted(int width, int height, int disparities) {
+static bool tiles_wanted(const PathSetup &s) {
     return g_path_tiles == 2 ||
-           (g_path_tiles == 1 && (size_t)width * height * disparities >= kTilesFrom);
+           (g_path_tiles == 1 && s.volume >= (s.paths == 8 ? 96 : 560) * kMi);
 }
 
 // The scan in the sweep order, one warp per block.
@@ -211,38 +213,63 @@ __global__ void __launch_bounds__(32)
                                    ring + threadIdx.x);
 }
 
-// Whether a pair's lines go in the sweep order: from 64 Mi pixel-disparities on (half the
-// L2), up to 128 disparities, where its warps of equal lines measured faster (us of the scan,
-// ranked lines or tiles -> sweep; 8 paths: 960x600x128 178 -> 163, 1024x768x96 214 -> 205,
-// 1024x768x128 252 -> 218, 1280x720x128 306 -> 277, 1600x1200x64 346 -> 286, 1600x900x128 465
-// -> 452, 1920x1080x128 695 -> 685; 3 paths: 1280x720x128 183 -> 171) and below it the ranked
-// ones, whose short lines fill the schedulers' gaps (1280x720x64 156 -> 170, 728x544x128 113
-// -> 119). With 16 lanes a line, two lines a warp make enough warps for the ranked lines and
-// the tile copies to balance, and the sweep is faster only at 192 disparities with 8 paths
-// from 160 Mi on (1280x720x192 491 -> 467, 1920x1080x192 1184 -> 1085; 800x600x192 233 -> 243),
-// at 256 with 3 paths (1280x720x256 283 -> 248), and with 8 by little from 256 to 768 Mi
-// (1280x720x256 578 -> 603, 1600x900x256 904 -> 900, 1920x1080x256 1333 -> 1321, 2560x1440x256
-// 2411 -> 2471): there the volume is read from memory once a direction in either order.
-constexpr size_t kMi = (size_t)1 << 20, kSweepFrom = 64 * kMi;
+// Whether a pair's lines go in the sweep order: where its warps of equal lines measured
+// faster, by the pair's pixel-disparities (us of the scan; ranked lines, or tiles where they
+// are the other choice -> sweep). Below each range the ranked lines' short diagonals fill the
+// schedulers' gaps, above it the tile copies read the costs at a higher rate.
+//   8 paths, 64 disparities, 96 to 360 Mi: 1440x810 (71 Mi) 182 -> 208, 1600x900 (88) 242 ->
+//   243, 1700x1000 (104) 292 -> 274, 1920x1080 362 -> 321, 3000x1900 (348) 1040 -> 978,
+//   3100x2000 (378) 1110 -> 1131, 3840x2160 (506) 1557 -> 1598; from 64 Mi where the columns
+//   are the longer lines: 900x1200 (66) 165 -> 162, 800x1500 292 -> 190, 900x1600 350 -> 219.
+//   96, from 64 Mi (no tiles): 1000x700 (64) 195 -> 204, 1200x800 (88) 278 -> 245, 1920x1080
+//   632 -> 586, 3840x2160 2768 -> 2568.
+//   128, 64 to 224 Mi: 960x600 178 -> 163, 1280x720 293 -> 270, 1600x1000 (195) 523 -> 494,
+//   1600x1100 (215) 568 -> 549, 1760x1000 (215) 564 -> 580, 1600x1200 (234) 614 -> 664,
+//   1920x1080 (253) 680 -> 681, 2560x1440 (450) 1287 -> 1363.
+//   160 to 224, from 160 Mi (no tiles): 800x600x192 (88) 233 -> 243, 1280x720x192 503 -> 471,
+//   1920x1080x192 1213 -> 1163, 3840x2160x192 5109 -> 4777, 1920x1080x224 1392 -> 1291.
+//   256 never (16 lanes a line leave the tiles warps enough): 1280x720 578 -> 603, 1400x800 700
+//   -> 722, 1600x900 908 -> 905, 1920x1080 1332 -> 1321, 2048x1400 1838 -> 1961.
+//   3 paths (its lines are alike in either order), 96, 336 to 704 Mi: 2600x1400 (333) 426 ->
+//   438, 2560x1440 (338) 460 -> 438, 3400x1900 (591) 913 -> 843, 3840x2160 (759) 1157 -> 1187;
+//   128, 448 to 768 Mi: 1280x720 141 -> 176, 2400x1440 (422) 452 -> 463, 2560x1440 (450) 505
+//   -> 499, 3200x1900 (742) 846 -> 828, 3840x2160 (1012) 1163 -> 1200; 256, 220 to 768 Mi:
+//   1200x740 (217) 227 -> 229, 1280x720 (225) 253 -> 244, 1920x1080 578 -> 549, 2200x1500
+//   (806) 900 -> 910; 64 never: 1920x1080 182 -> 215, 2560x1920 344 -> 395.
 static bool sweep_wanted(const PathSetup &s) {
-    if (g_path_tiles != 1 || s.volume < kSweepFrom) return false;
-    if (s.disparities <= 128) return true;
-    if (s.paths == 3) return s.disparities == 256;
-    return s.disparities == 256 ? s.volume >= 256 * kMi && s.volume < 768 * kMi
-                                : s.volume >= 160 * kMi;
+    if (g_path_tiles != 1) return false;
+    auto within = [&](size_t from, size_t below) {
+        return s.volume >= from * kMi && s.volume < below * kMi;
+    };
+    constexpr size_t any = SIZE_MAX / kMi;
+    const int D = s.disparities;
+    if (s.paths == 8) {
+        if (D <= 64) return within(s.height > s.width ? 64 : 96, 360);
+        if (D <= 96) return within(64, any);
+        if (D <= 128) return within(64, 224);
+        return D < 256 && within(160, any);
+    }
+    switch (D) {
+    case 96: return within(336, 704);
+    case 128: return within(448, 768);
+    case 256: return within(220, 768);
+    default: return false;
+    }
 }
 
-// Warps a wave of the sweep holds (22 blocks a SM under the matcher's L1 split). In one wave
-// the rows, the longest lines, come first; in more the lines that go down do, so that they go
-// together (1920x1080x192 1172 -> 1085 us, 1280x720x128 277 and 278).
-constexpr int kSweepWave = 22 * 148;
+// Warps from which the lines that go down come before the rows, so that they go together: a
+// line measured, not the warps that run at once (an SM takes 32 of them). Rows first -> lines
+// that go down first: 2,580 warps (1080x1920x128) 684 -> 718 us, 2,610 (1440x900x128) 398 ->
+// 398; 3,420 (1920x1080x128 and x96) 674 -> 682 and 594 -> 586, 3,672 (2048x1200x128) 859 ->
+// 840, 4,560 (1280x720x192) 510 -> 472, 6,840 (1920x1080x192) 1240 -> 1146.
+constexpr int kDownFirstFrom = 3300;
 
 template <int G, bool FULL>
 static cudaError_t launch_sweep(const uint8_t *costs, uint8_t *paths_out, const PathSetup &s,
                                 cudaStream_t stream) {
     const int warps = sweep_warps(s.width, s.height, s.paths, G);
     return launch_after(paths_sweep_kernel<G, FULL>, dim3(warps), dim3(32), 0, stream, costs,
-                        paths_out, s, warps > kSweepWave);
+                        paths_out, s, warps >= kDownFirstFrom);
 }
 
 unsigned path_wait_failures() {
@@ -335,7 +362,7 @@ static void launch_paths_in(const uint8_t *costs, uint8_t *paths_out, const Path
                      : launch_sweep<16, false>(costs, paths_out, s, stream);
             return;
         }
-        if (full && tiles_wanted(s.width, s.height, s.disparities) &&
+        if (full && tiles_wanted(s) &&
             encode_cost_maps(costs, s.width, s.height, s.disparities, &maps)) {
             // 16 KB of tiles a block: too few of them in the matcher's split.
 #define NXS_TILED(G)                                                                           \
