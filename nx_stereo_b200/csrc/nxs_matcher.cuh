@@ -414,10 +414,15 @@ __device__ __forceinline__ uint32_t mad_lo(uint32_t a, uint32_t b, uint32_t c) {
 // rounds of three shuffles (xor s, 2s, 3s) and one three-way min cover four
 // lanes at once, so 8 lanes take two dependent shuffle rounds instead of three
 // (728x544x128: 118.8 against 122.9 us); 16 lanes keep the four pairwise rounds
-// (1920x1080x256: six shuffles in two rounds measured 1.4% slower).
+// (1920x1080x256: six shuffles in two rounds measured 1.4% slower). A line of the
+// whole warp takes one reduction, for which v's halves must be alike (4 words a lane:
+// 728x544x256 416.5 us, 425.5 with five rounds; persistent batches of 8 pairs at 192
+// and 256 disparities 2,135 and 2,052, 2,301 and 2,174).
 template <int G>
 __device__ __forceinline__ uint32_t line_minimum(uint32_t v) {
-    if constexpr (G >= 16) {
+    if constexpr (G == 32) {  // both halves alike: one warp-wide reduction
+        return __reduce_min_sync(kFullMask, v);
+    } else if constexpr (G >= 16) {
 #pragma unroll
         for (int offset = G / 2; offset >= 1; offset /= 2)
             v = vmin2(v, __shfl_xor_sync(kFullMask, v, offset));
