@@ -119,7 +119,8 @@ cudaError_t launch_census_costs(const uint8_t *left, const uint8_t *right, int w
 // x 16 bytes; the per-lane ring of the other steps shares the first stage.
 // kPathRing: steps of costs a lane keeps in flight by its own copies. 12 cover the L2's
 // latency under the streaming stores (1277x713x192 with 3 paths 485 us a pair, 499 with 8;
-// 16 gave no more), at 6 KB of shared memory a block.
+// 16 gave no more), at 6 KB of shared memory a block; 8 with 16 words a lane, whose slots
+// are twice as large (728x544x64 197.6 us with 12, 191.2 with 8).
 constexpr int kPathRing = 12;
 
 template <int G, int WORDS, bool FULL, int SPAN, bool SUMS = false, bool TILES = false>
@@ -128,7 +129,7 @@ __global__ void __launch_bounds__(32)
                  const PathSetup s, const __grid_constant__ CostMaps maps) {
     using Piece = typename std::conditional<WORDS == 4, uint2, uint4>::type;
     constexpr int PIECES = WORDS == 16 ? 2 : 1;
-    constexpr int RING = TILES ? kPrefetch : kPathRing;
+    constexpr int RING = TILES || WORDS == 16 ? kPrefetch : kPathRing;
     constexpr int RING_BYTES = RING * PIECES * 32 * (int)sizeof(Piece);
     constexpr int TILE_BYTES = kTileStages * kPrefetch * 32 * 16;
     static_assert(!TILES || RING_BYTES <= TILE_BYTES / kTileStages, "the ring fits one stage");

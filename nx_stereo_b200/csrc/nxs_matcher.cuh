@@ -788,7 +788,9 @@ struct LineScan {
             // min(prev, neighbours + p1, m + p2) - m + cost: the sum is one three-input
             // add taken mod 2^32, whose halves neither borrow nor carry (t >= m in both).
             const uint32_t neighbour = vmin2(below[k], above[k]);
-            const uint32_t raised = add2(neighbour, p1x2);
+            // (integer adds stay in their halves too: at most 0x7FFF + 0x7FFF)
+            const uint32_t raised =
+                WORDS == 16 ? mad_lo(neighbour, one, p1x2) : add2(neighbour, p1x2);
             const uint32_t t = __vimin3_u16x2(r[k], raised, j2);
             r[k] = t + cost[k] + negm2;
         }
@@ -802,10 +804,16 @@ struct LineScan {
             }
         } else {
             // The bytes first, then a predicated store: a branch around the packing too
-            // costs every step its resolution.
+            // costs every step its resolution. With 16 words a lane the bytes of two pieces
+            // held for that, and f16x2 adds above, cost more than they give (728x544x128
+            // 329 us, 316 with the branch, the multiply-adds and a ring of 8).
 #pragma unroll
             for (int c = 0; c < PIECES; ++c) {
-                if constexpr (PIECE == 16)
+                if constexpr (WORDS == 16) {
+                    if (store)
+                        __stcs(reinterpret_cast<uint4 *>(dst + 16 * c),
+                               SPAN ? pack_run16(r + 8 * c, byte) : pack16(r + 8 * c));
+                } else if constexpr (PIECE == 16)
                     store16_if(store, dst + 16 * c,
                                SPAN ? pack_run16(r + 8 * c, byte) : pack16(r + 8 * c));
                 else
