@@ -57,7 +57,8 @@ typedef struct nxs_request nxs_request;
  * (lib/nx_stereo/matcher.ex:248-260, native/stereo_match/src/main.rs:21-38). */
 nxs_status nxs_create(int device, nxs_context **context, char *error, size_t error_len);
 
-/* Releases every segment and the context's device memory. */
+/* Releases every segment and the context's device memory, and what the device's
+ * small pool (nxs_quality_device) keeps and no call uses. */
 void nxs_destroy(nxs_context *context);
 
 /* The library's version string. */
@@ -509,7 +510,10 @@ nxs_status nxs_despeckle_depth_cloud_device(const float *d_disparity, uint32_t w
                                             void *stream);
 
 /* Stage.Quality's sums (lib/nx_stereo/diagnostics.ex:258-271), f32[5]; then
- * previous := disparity. */
+ * previous := disparity. The column sums' scratch (20 bytes a column) comes from
+ * a small stream-ordered pool of the library on the current device, which keeps
+ * up to 32 MiB between calls until a context on the device is destroyed; a
+ * captured call's from the graph. */
 nxs_status nxs_quality_device(const float *d_disparity, float *d_previous, uint32_t width,
                               uint32_t height, float *d_sums, void *stream);
 

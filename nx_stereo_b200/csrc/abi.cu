@@ -401,6 +401,34 @@ extern "C" nxs_status nxs_create(int device, nxs_context **context, char *error,
     return NXS_OK;
 }
 
+// The library's own stream-ordered pool on the current device, made on first use (make). It
+// keeps up to 32 MiB (the step a pool grows by) between calls, until nxs_destroy: the device's
+// default pool gives everything back at each synchronisation, so that a call after one maps
+// memory anew (a lone pass of the stages at 1280x720 took 690 us, 500 of them that).
+static cudaMemPool_t small_pool(bool make) {
+    constexpr int kDevices = 64;
+    static std::mutex lock;
+    static cudaMemPool_t pools[kDevices] = {};
+    int device = 0;
+    if (cudaGetDevice(&device) || device < 0 || device >= kDevices) return nullptr;
+    std::lock_guard<std::mutex> guard(lock);
+    if (make && !pools[device]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props)) {
+            cudaGetLastError();  // the call goes on with the device's pool
+            return nullptr;
+        }
+        uint64_t keep = 32u << 20;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        pools[device] = pool;
+    }
+    return pools[device];
+}
+
 extern "C" void nxs_destroy(nxs_context *c) {
     if (!c) return;
     cudaSetDevice(c->device);
@@ -412,6 +440,7 @@ extern "C" void nxs_destroy(nxs_context *c) {
     c->scratch.release();
     c->io.release();
     cudaStreamDestroy(c->stream);
+    if (cudaMemPool_t pool = small_pool(false)) cudaMemPoolTrimTo(pool, 0);
     delete c;
 }
 
@@ -1027,31 +1056,6 @@ extern "C" nxs_status nxs_despeckle_depth_cloud_device(
                : NXS_OK;
 }
 
-// The library's own stream-ordered pool on the current device, made on first use. It keeps
-// up to 32 MiB (the step a pool grows by) between calls: the device's default pool gives
-// everything back at each synchronisation, so that a call after one maps memory anew (a lone
-// pass of the stages at 1280x720 took 690 us, 500 of them that).
-static cudaMemPool_t small_pool() {
-    constexpr int kDevices = 64;
-    static std::mutex lock;
-    static cudaMemPool_t pools[kDevices] = {};
-    int device = 0;
-    if (cudaGetDevice(&device) || device < 0 || device >= kDevices) return nullptr;
-    std::lock_guard<std::mutex> guard(lock);
-    if (!pools[device]) {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        cudaMemPool_t pool = nullptr;
-        if (cudaMemPoolCreate(&pool, &props)) return nullptr;
-        uint64_t keep = 32u << 20;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        pools[device] = pool;
-    }
-    return pools[device];
-}
-
 extern "C" nxs_status nxs_quality_device(const float *d_disparity, float *d_previous,
                                          uint32_t width, uint32_t height, float *d_sums,
                                          void *stream) {
@@ -1063,7 +1067,7 @@ extern "C" nxs_status nxs_quality_device(const float *d_disparity, float *d_prev
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &capturing)) return NXS_CUDA_ERROR;
     const bool captured = capturing != cudaStreamCaptureStatusNone;
-    const cudaMemPool_t pool = captured ? nullptr : small_pool();
+    const cudaMemPool_t pool = captured ? nullptr : small_pool(true);
     const size_t bytes = sizeof(float) * 5 * width;
     void **to = reinterpret_cast<void **>(&columns);
     if (!pool ? cudaMallocAsync(to, bytes, s) : cudaMallocFromPoolAsync(to, bytes, pool, s))
