@@ -219,7 +219,7 @@ uint32_t nxs_path_sums(uint32_t width, uint32_t height, uint32_t disparities);
  * paths, from 560 Mi with 3, but where the lines go in the sweep order (every
  * line of a direction at the same image row), which only mode 1 takes, in a
  * range of sizes for each disparity and path count (from 64 Mi on at the
- * earliest; 8 paths at 256 and 3 at 64 and 192 disparities never).
+ * earliest; 3 paths at 64 and 192 disparities never).
  * A tuning knob for the whole library; results do not depend on it.
  * nxs_path_wait_failures: the path scans' waits on those copies that gave up
  * on the current device (each wait is bounded, about 1 s; 0 unless a copy

@@ -225,12 +225,16 @@ __global__ void __launch_bounds__(32)
 //   96, from 64 Mi (no tiles): 1000x700 (64) 195 -> 204, 1200x800 (88) 278 -> 245, 1920x1080
 //   632 -> 586, 3840x2160 2768 -> 2568.
 //   128, 64 to 224 Mi: 960x600 178 -> 163, 1280x720 293 -> 270, 1600x1000 (195) 523 -> 494,
-//   1600x1100 (215) 568 -> 549, 1760x1000 (215) 564 -> 580, 1600x1200 (234) 614 -> 664,
-//   1920x1080 (253) 680 -> 681, 2560x1440 (450) 1287 -> 1363.
+//   1600x1100 (215) 568 -> 549, 1760x1000 (215) 564 -> 580, 1600x1200 (234) 614 -> 660, 2560x1440
+//   (450) 1287 -> 1363; to 256 Mi where one side is half as long again as the other, which
+//   makes enough lines: 1920x1080 (253) 687 -> 679, 1280x1600 (250) 683 -> 701.
 //   160 to 224, from 160 Mi (no tiles): 800x600x192 (88) 233 -> 243, 1280x720x192 503 -> 471,
 //   1920x1080x192 1213 -> 1163, 3840x2160x192 5109 -> 4777, 1920x1080x224 1392 -> 1291.
-//   256 never (16 lanes a line leave the tiles warps enough): 1280x720 578 -> 603, 1400x800 700
-//   -> 722, 1600x900 908 -> 905, 1920x1080 1332 -> 1321, 2048x1400 1838 -> 1961.
+//   256, 320 to 600 Mi and no higher than wide, where alone the two are within 1% and two
+//   contexts at once are faster in the sweep (1920x1080 4,874 -> 4,516, 1600x900 3,333 ->
+//   3,101): 1280x720 (225) 578 -> 603, 1500x850 (311) 802 -> 824, 1600x900 (352) 910 -> 914,
+//   1920x1080 (506) 1348 -> 1339, 2048x1152 (576) 1496 -> 1480, 2048x1280 (640) 1667 -> 1715,
+//   1080x1920 1311 -> 1397.
 //   3 paths (its lines are alike in either order), 96, 336 to 704 Mi: 2600x1400 (333) 426 ->
 //   438, 2560x1440 (338) 460 -> 438, 3400x1900 (591) 913 -> 843, 3840x2160 (759) 1157 -> 1187;
 //   128, 448 to 768 Mi: 1280x720 141 -> 176, 2400x1440 (422) 452 -> 463, 2560x1440 (450) 505
@@ -247,8 +251,11 @@ static bool sweep_wanted(const PathSetup &s) {
     if (s.paths == 8) {
         if (D <= 64) return within(s.height > s.width ? 64 : 96, 360);
         if (D <= 96) return within(64, any);
-        if (D <= 128) return within(64, 224);
-        return D < 256 && within(160, any);
+        if (D <= 128) {
+            const int longer = std::max(s.width, s.height), shorter = std::min(s.width, s.height);
+            return within(64, 2 * longer >= 3 * shorter ? 256 : 224);
+        }
+        return D < 256 ? within(160, any) : s.width >= s.height && within(320, 600);
     }
     switch (D) {
     case 96: return within(336, 704);

@@ -31,11 +31,12 @@ ORDERS = [
     (900, 1200, 64, "sweep"), (1200, 900, 64, "ranked"), (3000, 1900, 64, "sweep"),
     (3840, 2160, 64, "tiles"), (990, 700, 96, "ranked"), (1000, 750, 96, "sweep"),
     (3840, 2160, 96, "sweep"), (728, 544, 128, "ranked"), (960, 600, 128, "sweep"),
-    (1600, 1000, 128, "sweep"), (1600, 1280, 128, "tiles"), (2560, 1440, 128, "tiles"),
+    (1600, 1000, 128, "sweep"), (1600, 1280, 128, "tiles"), (1920, 1080, 128, "sweep"),
+    (1080, 1920, 128, "sweep"), (1280, 1600, 128, "tiles"), (2560, 1440, 128, "tiles"),
     (800, 600, 192, "ranked"), (1280, 720, 192, "sweep"), (2560, 1440, 192, "sweep"),
     (1920, 1080, 160, "sweep"), (1920, 1080, 224, "sweep"), (640, 480, 256, "ranked"),
-    (1280, 720, 256, "tiles"), (1400, 800, 256, "tiles"), (1920, 1080, 256, "tiles"),
-    (2048, 1400, 256, "tiles"),
+    (1280, 720, 256, "tiles"), (1400, 800, 256, "tiles"), (1920, 1080, 256, "sweep"),
+    (1080, 1920, 256, "tiles"), (2048, 1400, 256, "tiles"),
 ]
 ORDERS_3 = [
     (1920, 1080, 64, "ranked"), (2560, 1920, 64, "ranked"), (3840, 2600, 64, "tiles"),
