@@ -372,7 +372,8 @@ static void launch_paths_in(const uint8_t *costs, uint8_t *paths_out, const Path
         }
         if (full && tiles_wanted(s) &&
             encode_cost_maps(costs, s.width, s.height, s.disparities, &maps)) {
-            // 16 KB of tiles a block: too few of them in the matcher's split.
+            // 16 KB of tiles a block: too few of them in the matcher's split. By default
+            // only 64, 128 and 256 disparities above the sweep's sizes come here.
 #define NXS_TILED(G)                                                                           \
     launch_alone(paths_kernel<G, 8, true, 16, false, true>, dim3(total), dim3(32), 0, stream, \
                  costs, paths_out, s, maps)

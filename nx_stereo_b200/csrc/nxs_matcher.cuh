@@ -380,14 +380,17 @@ __device__ __forceinline__ void census_costs_tile(const uint8_t *__restrict__ le
 //   m = min over d of prev,
 // which equals the reference's min(min(a, p2), min(a[d-1], a[d+1]) + p1) + C
 // with a = prev - m; its out-of-range neighbours (p2 - p1, so p2 once p1 is
-// added) never beat m + p2, so they read as +inf. Lanes past D hold +inf.
+// added) never beat m + p2, so they read as +inf. Lanes past D read the line's
+// first costs and hold values around kFar2: their jump costs kFar2, and what the
+// steps take from it (m) sums to at most what they add (C) and p2.
 // A path starts from zero where it enters the image, so its first step is C.
 //
 // A group of G lanes follows one line, each lane holding 2 * WORDS
-// disparities as u16x2 words (five integer instructions per word and step),
-// and a warp follows 32 / G lines in lockstep. Each lane copies its costs for the next kPrefetch - 1 steps into a shared
-// ring with cp.async while a step computes, and stores its path costs with
-// 16-byte stores.
+// disparities as u16x2 words (five instructions per word and step), and a warp
+// follows 32 / G lines in lockstep. Each lane copies its costs for the steps
+// ahead into a shared ring with cp.async while a step computes (RING slots:
+// kPrefetch, or as the kernel that follows the lines asks), and stores its path
+// costs with 16-byte stores. kPrefetch is also the steps of a tile (CostMaps).
 constexpr int kPrefetch = 8;
 
 struct PathSetup {
@@ -679,33 +682,8 @@ __host__ __device__ constexpr int sum_position(int disparities, int j) {
     return (j % 16 < 8 ? 0 : disparities / 2) + 8 * (j / 16) + j % 8;
 }
 
-// The lines of one warp: G lanes per line, WORDS (4, 8 or 16) u16x2 words,
-// so 2 x WORDS disparities, per lane. `ring` is this thread's first slot of
-// the warp's kPrefetch x THREADS slots of 2 x WORDS bytes. SPAN (8 or 16, at
-// most 2 x WORDS): costs and path costs are in the permuted order of
-// span_disparity, so within each run of SPAN disparities word k holds
-// disparities (k, k + SPAN / 2) and its neighbours at d - 1 and d + 1 are the
-// words k - 1 and k + 1, but for the first and last word of a run, whose
-// outer neighbour lies in the next run (one byte permute each); SPAN 0:
-// word k holds (2k, 2k + 1) and every neighbour is made by a byte permute.
-//
-// SUMS: instead of its own u8 volume, each direction adds its path costs into
-// one u16 aggregate volume (zeroed before the launch) in the lane-split
-// layout of sum_position, with 16-byte reductions: every direction's lane
-// sends its words 0-3 and 4-7 as two reductions, so G lanes cover two runs of
-// 16 * G contiguous bytes. The reductions are f16x2 adds on the u16 bit
-// patterns: an integer n < 1024 is the f16 subnormal n * 2^-24, and the sum
-// of subnormals below 2^-14 is exact with subnormals kept (.noftz), so the
-// adds are the integer adds (8 directions x at most 127 = 1016).
-//
-// TILES (8 words a lane, span 16, every lane active): the blocks of 8 steps
-// that every line of the warp covers take their costs from bulk tensor copies
-// (CostMaps) instead of per-lane copies: one lane of each line asks for a
-// block's [8][D] tile kTileStages - 1 blocks ahead into a stage of `tiles`,
-// each stage completing on its own barrier of `bars` (LINES arrivals a
-// phase); the other blocks (each line's last ones) keep the per-lane copies,
-// their ring in the first stage's room once every tile has been read.
-// The state of one scan line as a lane holds it, and its step.
+// The state of one scan line as a lane holds it, and its step (the parameters are
+// follow_lines's).
 template <int G, int WORDS, bool FULL, int SPAN, bool SUMS>
 struct LineScan {
     static constexpr int RUN = SPAN / 2;  // words of a permuted run
@@ -824,6 +802,32 @@ struct LineScan {
     }
 };
 
+// The lines of one warp: G lanes per line, WORDS (4, 8 or 16) u16x2 words,
+// so 2 x WORDS disparities, per lane. `ring` is this thread's first slot of
+// the warp's RING x THREADS slots of 2 x WORDS bytes. SPAN (8 or 16, at
+// most 2 x WORDS): costs and path costs are in the permuted order of
+// span_disparity, so within each run of SPAN disparities word k holds
+// disparities (k, k + SPAN / 2) and its neighbours at d - 1 and d + 1 are the
+// words k - 1 and k + 1, but for the first and last word of a run, whose
+// outer neighbour lies in the next run (one byte permute each); SPAN 0:
+// word k holds (2k, 2k + 1) and every neighbour is made by a byte permute.
+//
+// SUMS: instead of its own u8 volume, each direction adds its path costs into
+// one u16 aggregate volume (zeroed before the launch) in the lane-split
+// layout of sum_position, with 16-byte reductions: every direction's lane
+// sends its words 0-3 and 4-7 as two reductions, so G lanes cover two runs of
+// 16 * G contiguous bytes. The reductions are f16x2 adds on the u16 bit
+// patterns: an integer n < 1024 is the f16 subnormal n * 2^-24, and the sum
+// of subnormals below 2^-14 is exact with subnormals kept (.noftz), so the
+// adds are the integer adds (8 directions x at most 127 = 1016).
+//
+// TILES (8 words a lane, span 16, every lane active): the blocks of 8 steps
+// that every line of the warp covers take their costs from bulk tensor copies
+// (CostMaps) instead of per-lane copies: one lane of each line asks for a
+// block's [8][D] tile kTileStages - 1 blocks ahead into a stage of `tiles`,
+// each stage completing on its own barrier of `bars` (LINES arrivals a
+// phase); the other blocks (each line's last ones) keep the per-lane copies,
+// their ring in the first stage's room once every tile has been read.
 template <int G, int WORDS, bool FULL, int THREADS, int SPAN = 0, bool SUMS = false,
           bool TILES = false, int RING = kPrefetch>
 __device__ __forceinline__ void follow_lines(const uint8_t *__restrict__ costs,
@@ -1003,7 +1007,7 @@ __host__ __device__ __forceinline__ int ranked_line(int rank, int dy, int dx, in
 
 // One warp's lines: warp `warp` of the pair's path launch, lane `lane`.
 // Rows, then columns, then the diagonals of all four directions by rank.
-// `ring`: this lane's first slot of the warp's kPrefetch x 32 slots of
+// `ring`: this lane's first slot of the warp's RING x 32 slots of
 // 2 x WORDS bytes (in pieces of at most 16 bytes, strided by 32 lanes).
 template <int G, int WORDS, bool FULL, int SPAN = 0, bool SUMS = false, bool TILES = false,
           int RING = kPrefetch>
